@@ -104,7 +104,9 @@ typedef struct {
     int32_t small_path;      /* 1: tsg_spgemm runs A*B and A*A whose every row of A meets at most 128 entries of B
                                 (A and B of at most 4 M entries) row by row, one warp per row of C, instead of
                                 the tiled pipeline -- the same C, values included; a repeated shape waits on the
-                                device once per call; 0: always the tiled pipeline (default 1) */
+                                device once per call.  Products without statistics (stats NULL) that are small, or
+                                whose tiles would be nearly empty, and B's rows increase strictly, also run row by
+                                row, a warp or CTA per part of a row; 0: always the tiled pipeline (default 1) */
 } tsg_opts;
 
 /* Per-call statistics.  Sizes are always filled; times only with phase_times. */

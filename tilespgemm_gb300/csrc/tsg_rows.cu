@@ -1,0 +1,746 @@
+// tsg_rows.cu -- the row path of tsg_spgemm: C = A*B row by row for products
+// whose 16x16 tiles are nearly empty (graphs, unstructured matrices).
+//
+// A tile of such a matrix holds one to three entries, so tile masks move 16
+// halfwords for each of them, a hub's tile-row is one CTA's work, and its
+// wide rows accumulate in C itself.  Here a row of C is cut into *items* by
+// its own entries, each one warp's or one CTA's work anywhere on the GPU:
+//   k_row_sample    the products of every 16th row (the choice of the path)
+//   k_row_extents / k_row_products   per row of C its products and the blocks
+//                   of ROW_BLK columns it can reach; heavy rows listed by
+//                   weight, so that the longest chains start first
+//   k_row_cuts      per row of B the first entry at or past every block (the
+//                   cut table), when a row of C has several items
+//   k_row_symbolic  per row of C a bitmap of its columns in shared memory, its
+//                   entries per block, and from them its items: one for a
+//                   light row, else runs of blocks that close at ITEM_T
+//                   entries or ITEM_BLKS blocks
+//   (the look-back scan of the row counts gives C's row pointer)
+//   k_row_numeric   per item: the bitmap of its columns and running counts (a
+//                   column's position = count + popc), then its products in
+//                   steps, one A entry's B entries each: one fma a product on
+//                   its position's accumulator in shared memory
+// The steps follow one another in A's row order and a step's columns differ,
+// so every entry of C sees fma(a_ik, b_kj, c) over k in A's row order, from
+// 0.0, as in the tiled kernels and the oracle: the values are the same bits.
+// B's rows must be strictly increasing (checked on the device by
+// k_count_descents; the tiled path takes the others).
+//
+// Measured on GB300, before (tiled) and after, whole call on the device:
+//   R-MAT 2^12 x 8 A*A^T 1,190 -> 431 us, 2^15 x 16 A*A^T 8.4 -> 2.3 ms,
+//   2^16 x 12 A*A 12.9 -> 3.4 ms, 2^18 x 16 A*A^T 80 -> 42 ms;
+//   uniform 120,007 x 80,021 x 100,003, 16 and 12 a row: 10.3 -> 2.0 ms.
+// What bounds it (2^15, counters): k_row_numeric, 2/3 of the time, is bound
+// by issue and by the latency of a step's chain (B's entry, its word, its
+// accumulator, the fma): some 60 instructions a step at 1.1 to 1.6 a clock
+// and SM, FP64 pipe 20-30 % busy.  k_row_symbolic is bound by its bitmap's
+// shared-memory accesses.
+// Tried without gain: products flattened 32 at a time over an item's shares,
+// lanes that meet ordered by rank (2^18: 77 ms; R-MAT's columns meet in
+// nearly every round); items of 6,144 entries as a CTA's, 128 entries a step
+// (67 ms: idle warps and a barrier a step); groups of 2 or 8 steps in flight
+// in place of 4 (50 / 58 against 45 ms: loads exposed, code outgrows the
+// instruction cache).
+// The reference bins C's rows by intermediate products for its tile-level
+// symbolic step (spgemm_nsparse_kernel.h:32-311); it has no row path.
+#include "tsg_internal.cuh"
+#include "tsg_rows.cuh"
+
+#include <algorithm>
+#include <climits>
+
+namespace tsg {
+
+namespace {
+
+constexpr unsigned FULL = 0xffffffffu;
+// The products of every step-th row of C, times step (one warp a row).
+__global__ void __launch_bounds__(256)
+k_row_sample(RowArgs g, int step, unsigned long long *out)
+{
+    const long long r = (blockIdx.x * 8ll + (threadIdx.x >> 5)) * step;
+    if (r >= g.m) return;
+    long long p = 0;
+    for (long long e = g.rpA[r] + (threadIdx.x & 31); e < g.rpA[r + 1]; e += 32) {
+        const int k = g.colA[e];
+        if ((unsigned)k < (unsigned)g.k) p += g.rpB[k + 1] - g.rpB[k];
+    }
+    p = warp_sum_ll(p);
+    if ((threadIdx.x & 31) == 0 && p) atomicAdd(out, (unsigned long long)(p * step));
+}
+
+// Per row of B its first and last block of columns (one thread each).
+__global__ void k_row_extents(const long long *__restrict__ rpB, const int *__restrict__ colB, int kB, int2 *ext)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= kB) return;
+    const long long s = rpB[k], e = rpB[k + 1];
+    ext[k] = e > s ? make_int2(colB[s] >> ROW_BLK_LOG, colB[e - 1] >> ROW_BLK_LOG) : make_int2(INT_MAX, -1);
+}
+
+// Per row of C (one warp each): its products, INT_MAX at most, and its blocks
+// [x, y); rows of more than ROW_HEAVY products are listed by weight.
+__global__ void __launch_bounds__(256)
+k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, int *heavy, RowStat *stat)
+{
+    __shared__ unsigned long long s_p[8], s_i[8];
+    __shared__ int s_w[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned long long sp = 0, si = 0;
+    int width = 0;
+    for (long long r = blockIdx.x * 8ll + warp; r < g.m; r += gridDim.x * 8ll) {
+        long long p = 0;
+        int lo = INT_MAX, hi = -1;
+        bool out = false;
+        const long long e1 = g.rpA[r + 1];
+        for (long long e = g.rpA[r] + lane; e < e1; e += 128) {
+            int k[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) k[u] = e + 32 * u < e1 ? g.colA[e + 32 * u] : -1;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if ((unsigned)k[u] < (unsigned)g.k) {
+                    p += g.rpB[k[u] + 1] - g.rpB[k[u]];
+                    const int2 x = ext[k[u]];
+                    lo = min(lo, x.x);
+                    hi = max(hi, x.y);
+                } else if (e + 32 * u < e1) {
+                    out = true;
+                }
+            }
+        }
+        p = warp_sum_ll(p);
+        lo = __reduce_min_sync(FULL, lo);
+        hi = __reduce_max_sync(FULL, hi);
+        if (out) stat->bad = 1;
+        if (lane == 0) {
+            prod[r] = (int)min(p, (long long)INT_MAX);
+            const int nb = hi < lo ? 0 : hi - lo + 1;
+            rng[r] = make_int2(nb ? lo : 0, nb ? hi + 1 : 0);
+            width = max(width, nb);
+            sp += (unsigned long long)p;
+            si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
+            if ((p > LIGHT_ROW || nb > SYM_BLKS) && !stat->cuts) stat->cuts = 1;
+            if (p > ROW_HEAVY) {
+                const int c = heavy_class(p);
+                heavy[(long long)c * g.m + atomicAdd(stat->heavy + c, 1u)] = (int)r;
+            }
+        }
+    }
+    if (lane == 0) { s_p[warp] = sp; s_i[warp] = si; s_w[warp] = width; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long a = 0, b = 0;
+        int w = 0;
+        for (int q = 0; q < 8; ++q) { a += s_p[q]; b += s_i[q]; w = max(w, s_w[q]); }
+        atomicAdd(&stat->products, a);
+        atomicAdd(&stat->items, b);
+        if (w > *(volatile int *)&stat->width) atomicMax(&stat->width, w);
+    }
+}
+
+// Row k of the cut table (one warp each): cut[k][j] = B's first entry of row
+// k at column j * ROW_BLK or past it; j = 0..nblk.  Written coalesced, read
+// back by k_row_numeric as two neighbouring ints per A entry and item.
+__global__ void __launch_bounds__(256)
+k_row_cuts(const long long *__restrict__ rpB, const int *__restrict__ colB, int kB, int nblk, int *__restrict__ cut)
+{
+    const long long k = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (k >= kB) return;
+    const int b0 = (int)rpB[k], b1 = (int)rpB[k + 1];
+    int *row = cut + k * (nblk + 1);
+    for (int j = lane; j <= nblk; j += 32) {
+        int a = b0, b = b1;
+        if (j == nblk) a = b1;
+        else {
+            const int key = j << ROW_BLK_LOG;
+            while (a < b) {
+                const int md = (a + b) >> 1;
+                if (colB[md] < key) a = md + 1; else b = md;
+            }
+        }
+        row[j] = a;
+    }
+}
+
+// The heavy rows' lists (HEAVY_CLASSES of m), the heaviest class last.
+struct HeavyRows {
+    const int *list = nullptr;
+    int n[HEAVY_CLASSES] = {};
+    long long m = 0;
+    __device__ int row(int i) const {
+        int c = HEAVY_CLASSES - 1;
+        while (c > 0 && i >= n[c]) i -= n[c--];
+        return list[c * m + i];
+    }
+};
+
+// One CTA per row of C with products in (p0, p1]: the row's columns as a
+// bitmap of up to SYM_BLKS blocks at a time in shared memory, then its entry
+// count and its items.  heavy.list: those rows, the heaviest first; without a
+// list the grid is all rows (rows of no product belong to p0 = 0).
+template <int NT>
+__global__ void __launch_bounds__(NT)
+k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRows heavy, int width, int *rowcnt,
+               int4 *items, unsigned cap, unsigned *nitems)
+{
+    constexpr int NW = NT / 32;
+    extern __shared__ __align__(16) unsigned s_sym[];
+    const int r = heavy.list ? heavy.row(blockIdx.x) : blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int p = prod[r];
+    if (p <= p0 || p > p1) {
+        if (p == 0 && p0 == 0 && tid == 0) rowcnt[r] = 0;
+        return;
+    }
+    // the row's blocks: first, then counted from it
+    const int2 rng = g.rng[r];
+    const int first = rng.x, nblk = rng.y - rng.x;
+    unsigned *bits = s_sym;
+    int *cnt = reinterpret_cast<int *>(s_sym + min(width, SYM_BLKS) * (ROW_BLK / 32));
+    const long long a0 = g.rpA[r], a1 = g.rpA[r + 1];
+    for (int wb = 0; wb < nblk; wb += SYM_BLKS) {
+        const int nb = min(SYM_BLKS, nblk - wb);
+        const int c0 = (first + wb) << ROW_BLK_LOG;
+        {
+            uint4 *z = reinterpret_cast<uint4 *>(bits);
+            for (int t = tid; t < nb * (ROW_BLK / 128); t += NT) z[t] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        auto mark = [&](int c) {      // most columns of a long row are met before: the atomic is left out
+            const int o = c - c0;
+            const unsigned bit = 1u << (o & 31);
+            volatile unsigned *w = bits + (o >> 5);
+            if (!(*w & bit)) atomicOr(bits + (o >> 5), bit);
+        };
+        auto share = [&](long long a, int &s, int &e) {
+            s = e = 0;
+            if (a < a1) {
+                const int k = g.colA[a];
+                if (nblk <= SYM_BLKS) { s = (int)g.rpB[k]; e = (int)g.rpB[k + 1]; }
+                else {
+                    const int *row = g.cut + (long long)k * (g.nblk + 1) + first + wb;
+                    s = row[0];
+                    e = row[nb];
+                }
+            }
+        };
+        auto range = [&](int t, int e, int step) {   // entries t, t + step, ... below e, four on their way
+            for (; t + 3 * step < e; t += 4 * step) {
+                const int x0 = g.colB[t], x1 = g.colB[t + step], x2 = g.colB[t + 2 * step], x3 = g.colB[t + 3 * step];
+                mark(x0); mark(x1); mark(x2); mark(x3);
+            }
+            for (; t < e; t += step) mark(g.colB[t]);
+        };
+        if (a1 - a0 > 4 * NW) {
+            // many A entries: warp w takes those at w, w + NW, ... (the hubs'
+            // long B rows lie side by side), four shares on their way
+            for (long long a = a0 + warp; a < a1; a += 32 * NW) {
+                int s, e;
+                share(a + (long long)lane * NW, s, e);
+                unsigned live = __ballot_sync(FULL, e > s);
+                while (live) {
+                    int sq[4], eq[4], c[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int q = live ? __ffs(live) - 1 : 0;
+                        sq[u] = __shfl_sync(FULL, s, q);
+                        eq[u] = live ? __shfl_sync(FULL, e, q) : sq[u];
+                        live &= live - 1;
+                        c[u] = sq[u] + lane < eq[u] ? g.colB[sq[u] + lane] : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (c[u] >= 0) mark(c[u]);
+                        range(sq[u] + 32 + lane, eq[u], 32);
+                    }
+                }
+            }
+        } else {
+            for (long long a = a0; a < a1; a += 32) {
+                int s, e;
+                share(a + lane, s, e);
+                // long B rows are the whole CTA's, the others a warp's each
+                unsigned big = __ballot_sync(FULL, e - s > 64 * NW);
+                unsigned small = __ballot_sync(FULL, e > s) & ~big;
+                while (big) {
+                    const int q = __ffs(big) - 1;
+                    big &= big - 1;
+                    range(__shfl_sync(FULL, s, q) + tid, __shfl_sync(FULL, e, q), NT);
+                }
+                for (int turn = 0; small; ++turn) {
+                    const int q = __ffs(small) - 1;
+                    small &= small - 1;
+                    const int sq = __shfl_sync(FULL, s, q), eq = __shfl_sync(FULL, e, q);
+                    if ((turn & (NW - 1)) == warp) range(sq + lane, eq, 32);
+                }
+            }
+        }
+        __syncthreads();
+        for (int j = warp; j < nb; j += NW) {
+            const unsigned c = __reduce_add_sync(FULL, (unsigned)__popc(bits[j * (ROW_BLK / 32) + lane]));
+            if (lane == 0) cnt[wb + j] = (int)c;
+        }
+        __syncthreads();
+    }
+    if (warp != 0) return;
+    // the items: block j starts one when it is a multiple of ITEM_BLKS or the
+    // entries before it have passed another multiple of ITEM_T (light rows:
+    // every LIGHT_BLKS blocks only); a start closes the item before it.  Two passes: the items of each class counted, then
+    // written where the row's share of the class's list begins.
+    __shared__ unsigned s_cls[ITEM_CLASSES];
+    const long long la = a1 - a0;
+    int tclose = ITEM_T, bmax = ITEM_BLKS;      // a row's items close at so many entries, or blocks
+    auto close = [&](int j, int e, int pj, int pe, bool write) {   // blocks [pj, j), entries [pe, e) of the row
+        const int z = e - pe, nb = j - pj;
+        if (z <= 0) return;
+        const int c = item_class(z, nb, (float)p * (float)z / ((float)la * (float)cnt[nblk]), tclose > ITEM_T);
+        const unsigned i = atomicAdd(s_cls + c, 1u);
+        if (write && i < cap) items[(unsigned long long)c * cap + i] = make_int4(r, first + pj, pe, (nb << 16) | z);
+    };
+    auto pass = [&](bool write) -> int {
+        int run = 0, pj = 0, pe = 0;
+        for (int jb = 0; jb < nblk; jb += 32) {
+            const int j = jb + lane;
+            const int c = j < nblk ? cnt[j] : 0;
+            const int incl = warp_incl_scan(c, lane);
+            const int excl = run + incl - c;
+            int before = __shfl_up_sync(FULL, excl, 1);
+            if (lane == 0) before = run - (jb > 0 ? cnt[jb - 1] : 0);
+            const bool st = j < nblk && j > 0 && (j % bmax == 0 || excl / tclose != before / tclose);
+            const unsigned starts = __ballot_sync(FULL, st);
+            const unsigned lower = starts & lanemask_lt();
+            const int q = 31 - __clz(lower);
+            const int qe = __shfl_sync(FULL, excl, q & 31);
+            if (st) close(j, excl, lower ? jb + q : pj, lower ? qe : pe, write);
+            if (starts) {
+                const int last = 31 - __clz(starts);
+                pj = jb + last;
+                pe = __shfl_sync(FULL, excl, last);
+            }
+            run += __shfl_sync(FULL, incl, 31);
+        }
+        if (lane == 0) {
+            close(nblk, run, pj, pe, write);
+        }
+        __syncwarp();
+        return run;
+    };
+    {   // the row's entries, which the classes go by
+        int t = 0;
+        for (int j = lane; j < nblk; j += 32) t += cnt[j];
+        t = warp_sum_int(t);
+        if (lane == 0) { cnt[nblk] = t; rowcnt[r] = t; }
+        if (t <= LIGHT_ROW) { tclose = LIGHT_ROW + 1; bmax = LIGHT_BLKS; }
+        __syncwarp();
+    }
+    if (cnt[nblk] <= LIGHT_ROW && nblk <= LIGHT_BLKS) {      // one item
+        const int z = cnt[nblk];
+        if (lane == 0 && z > 0) {
+            const int c = item_class(z, nblk, (float)p / (float)la, true);
+            const unsigned i = atomicAdd(nitems + c, 1u);
+            if (i < cap) items[(unsigned long long)c * cap + i] = make_int4(r, first, 0, (nblk << 16) | z);
+        }
+        return;
+    }
+    if (lane < ITEM_CLASSES) s_cls[lane] = 0;
+    __syncwarp();
+    pass(false);
+    if (lane < ITEM_CLASSES) {
+        const unsigned mine = s_cls[lane];
+        s_cls[lane] = mine ? atomicAdd(nitems + lane, mine) : 0u;
+    }
+    __syncwarp();
+    pass(true);
+}
+
+struct __align__(16) Step {  // up to NT of one A entry's products: B's entries at..last
+    int at, last;
+    double a;
+};
+
+// One item, one CTA.  Its products come in steps of up to NT entries of one
+// A entry's B row: the threads' columns differ, so a step is one fma per
+// position, and the steps follow one another in A's order, a barrier between
+// them.  A step's idle lanes repeat its last entry and keep the result to
+// themselves; warps without a product only meet the barrier.
+template <int NT>
+__global__ void __launch_bounds__(NT)
+k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__restrict__ rowptrC,
+              int *__restrict__ colC, double *__restrict__ valC, int *flags)
+{
+    constexpr int NW = NT / 32, STEPS = row_steps(NT);
+    extern __shared__ __align__(16) unsigned char s_num[];
+    __shared__ int s_sum[NW + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto sync = [] { if constexpr (NT > 32) __syncthreads(); else __syncwarp(); };
+    const int4 it = items[blockIdx.x];
+    const int r = it.x, j0 = it.y, z = it.w & 0xffff, nb = it.w >> 16;
+    const int c0 = j0 << ROW_BLK_LOG, nw = nb * (ROW_BLK / 32);
+    const bool dense = item_dense(z, nb);
+    Step *steps = reinterpret_cast<Step *>(s_num);
+    uint2 *word = reinterpret_cast<uint2 *>(steps + STEPS);                     // column bits, entries before them
+    unsigned char *tag = reinterpret_cast<unsigned char *>(steps + STEPS);     // dense items: the columns met
+    double *acc = reinterpret_cast<double *>(tag + (dense ? nb * ROW_BLK : nw * 8));
+    int *ccol = reinterpret_cast<int *>(acc + z);      // ranked items of many blocks: the positions' columns
+    const bool wide = nb > ITEM_BLKS;
+    const long long a0 = g.rpA[r], a1 = g.rpA[r + 1];
+    const int2 rng = g.rng[r];
+    const bool whole = nb == rng.y - rng.x;      // the row's only item: whole B rows
+    for (int w = tid; w < (dense ? nb * (ROW_BLK / 16) : nw / 2); w += NT)
+        reinterpret_cast<uint4 *>(tag)[w] = make_uint4(0u, 0u, 0u, 0u);
+    for (int t = tid; t < (dense ? nb * ROW_BLK : z); t += NT) acc[t] = 0.0;
+    int nk = -1, ns = 0, ne = 0;       // the next NT A entries' B rows and shares, loaded ahead
+    double nav = 0.0;
+    auto load_k = [&](long long a) { nk = a + tid < a1 ? g.colA[a + tid] : -1; };
+    auto load_share = [&](long long a) {
+        ns = ne = 0;
+        if (nk >= 0) {
+            nav = g.valA[a + tid];
+            if (whole) { ns = (int)g.rpB[nk]; ne = (int)g.rpB[nk + 1]; }
+            else {
+                const int *row = g.cut + (long long)nk * (g.nblk + 1) + j0;
+                ns = row[0];
+                ne = row[nb];
+            }
+        }
+    };
+    // f(number of steps staged) over all of the item's steps; the list is
+    // filled up to a multiple of ROW_GROUP with steps without entries
+    auto walk = [&](auto f) {
+        load_k(a0);
+        load_share(a0);
+        load_k(a0 + NT);
+        for (long long a = a0; a < a1; a += NT) {
+            const int s = ns, e = ne;
+            const double av = nav;
+            load_share(a + NT);
+            load_k(a + 2 * NT);
+            const int cnt = (e - s + NT - 1) / NT;
+            int incl = warp_incl_scan(cnt, lane), total = __shfl_sync(FULL, incl, 31);
+            if constexpr (NT > 32) {
+                __syncthreads();
+                if (lane == 0) s_sum[warp] = total;
+                __syncthreads();
+                total = 0;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    if (w < warp) incl += s_sum[w];
+                    total += s_sum[w];
+                }
+            }
+            for (int base = 0; base < total; base += STEPS) {
+                const int at = incl - cnt - base;            // of this thread's first step
+                const int n = min(STEPS, total - base);
+                sync();
+                for (int q = max(0, -at); q < cnt && at + q < STEPS; ++q) {
+                    const int last = min(s + NT * q + NT, e) - 1;
+                    steps[at + q] = Step{s + NT * q, last, av};
+                    if (at + q == n - 1)
+                        for (int w = n; w & (ROW_GROUP - 1); ++w) steps[w] = Step{last + 1, last, 0.0};
+                }
+                sync();
+                f(n);
+            }
+        }
+        sync();
+    };
+    if (!dense) {
+        // the columns: a warp takes every NW-th group of steps, or, with
+        // steps wider than a warp, every NW-th step
+        walk([&](int n) {
+            auto mark = [&](int c) { atomicOr(&word[(c - c0) >> 5].x, 1u << (c & 31)); };
+            if constexpr (NT == 32) {
+                for (int i = 0; i < n; i += ROW_GROUP) {
+                    int c[ROW_GROUP];
+                    bool live[ROW_GROUP];
+#pragma unroll
+                    for (int u = 0; u < ROW_GROUP; ++u) {
+                        const int t = steps[i + u].at + lane;
+                        live[u] = t <= steps[i + u].last;
+                        c[u] = live[u] ? g.colB[t] : 0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < ROW_GROUP; ++u)
+                        if (live[u]) mark(c[u]);
+                }
+            } else {
+                for (int i = warp; i < n; i += NW) {
+                    const int last = steps[i].last;
+                    int c[NW];
+#pragma unroll
+                    for (int u = 0; u < NW; ++u) {
+                        const int t = steps[i].at + 32 * u + lane;
+                        c[u] = t <= last ? g.colB[t] : -1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < NW; ++u)
+                        if (c[u] >= 0) mark(c[u]);
+                }
+            }
+        });
+        // the entries before each word: a warp takes a run of words, 64 a
+        // round; then the warps' totals
+        const int per = ((nw + NW - 1) / NW + 63) & ~63, w1 = min(nw, (warp + 1) * per);
+        int run = 0;
+        for (int w = warp * per + 2 * lane; w - 2 * lane < w1; w += 64) {
+            uint4 x = w < w1 ? *reinterpret_cast<const uint4 *>(word + w) : make_uint4(0u, 0u, 0u, 0u);
+            const int n0 = __popc(x.x), sum = n0 + __popc(x.z);
+            const int incl = warp_incl_scan(sum, lane);
+            x.y = (unsigned)(run + incl - sum);
+            x.w = x.y + (unsigned)n0;
+            run += __shfl_sync(FULL, incl, 31);
+            if (w < w1) *reinterpret_cast<uint4 *>(word + w) = x;
+        }
+        int total = run;
+        if constexpr (NT > 32) {
+            if (lane == 0) s_sum[warp] = run;
+            __syncthreads();
+            int base = 0;
+            total = 0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                if (w < warp) base += s_sum[w];
+                total += s_sum[w];
+            }
+            if (base)
+                for (int w = warp * per + lane; w < w1; w += 32) word[w].y += (unsigned)base;
+        }
+        sync();
+        if (total != z) {
+            if (tid == 0) set_flag(flags, FLAG_INTERNAL);
+            return;
+        }
+    }
+    // the values: two groups of steps, one's entries loaded while the other's
+    // are applied
+    auto values = [&](auto position) {
+        walk([&](int n) {
+            struct Group {
+                int col[ROW_GROUP];
+                bool live[ROW_GROUP], on[ROW_GROUP];
+                double b[ROW_GROUP], a[ROW_GROUP];
+            } x, y;
+            auto load = [&](int i, Group &v) {
+                if (i >= n) return;
+#pragma unroll
+                for (int u = 0; u < ROW_GROUP; ++u) {
+                    const Step q = steps[i + u];
+                    const int t = q.at + tid;
+                    v.live[u] = t <= q.last;
+                    v.on[u] = NT == 32 || q.at + warp * 32 <= q.last;
+                    if (v.on[u]) {
+                        const int e = min(t, q.last);
+                        v.col[u] = g.colB[e];
+                        v.b[u] = g.valB[e];
+                        v.a[u] = q.a;
+                    }
+                }
+            };
+            auto apply = [&](int i, const Group &v) {
+                if (i >= n) return;
+                int p[ROW_GROUP];
+#pragma unroll
+                for (int u = 0; u < ROW_GROUP; ++u)
+                    if (v.on[u]) p[u] = position(v.col[u], v.live[u]);
+#pragma unroll
+                for (int u = 0; u < ROW_GROUP; ++u) {
+                    if (v.on[u]) {
+                        const double c = fma(v.a[u], v.b[u], acc[p[u]]);
+                        if (v.live[u]) acc[p[u]] = c;
+                    }
+                    sync();
+                }
+            };
+            load(0, x);
+            load(ROW_GROUP, y);
+            for (int i = 0; i < n; i += 2 * ROW_GROUP) {
+                apply(i, x);
+                load(i + 2 * ROW_GROUP, x);
+                apply(i + ROW_GROUP, y);
+                load(i + 3 * ROW_GROUP, y);
+            }
+        });
+    };
+    const long long Rb = rowptrC[r] + it.z;
+    if (dense) {
+        values([&](int c, bool live) {
+            const int o = live ? c - c0 : 0;
+            if (live) tag[o] = 1;
+            return o;
+        });
+        // a word's columns a round; a warp takes a run of words, counted first
+        const int per = (nw + NW - 1) / NW, w0 = warp * per, w1 = min(nw, w0 + per);
+        int run = 0, total = 0;
+        if constexpr (NT > 32) {
+            int c = 0;
+            for (int w = w0; w < w1; ++w) c += tag[w * 32 + lane];
+            c = (int)__reduce_add_sync(FULL, (unsigned)c);
+            if (lane == 0) s_sum[warp] = c;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                if (w < warp) run += s_sum[w];
+                total += s_sum[w];
+            }
+            if (total != z) {
+                if (tid == 0) set_flag(flags, FLAG_INTERNAL);
+                return;
+            }
+        }
+#pragma unroll 4
+        for (int w = w0; w < w1; ++w) {
+            const bool met = tag[w * 32 + lane] != 0;
+            const unsigned m = __ballot_sync(FULL, met);
+            const int t = run + __popc(m & lanemask_lt());
+            if (met && t < z) {
+                valC[Rb + t] = acc[w * 32 + lane];
+                colC[Rb + t] = c0 + w * 32 + lane;
+            }
+            run += __popc(m);
+        }
+        if (NT == 32 && run != z && lane == 0) set_flag(flags, FLAG_INTERNAL);
+        return;
+    }
+    const uint2 *word0 = word - (c0 >> 5);
+    auto rank = [&](int c) {
+        const uint2 w = word0[c >> 5];
+        return (int)w.y + __popc(w.x & ((1u << (c & 31)) - 1u));
+    };
+    if (wide) {
+        values([&](int c, bool live) {
+            const int pos = rank(c);
+            if (live) ccol[pos] = c;
+            return pos;
+        });
+    } else {
+        values([&](int c, bool) { return rank(c); });
+    }
+    for (int t = tid; t < z; t += NT) valC[Rb + t] = acc[t];
+    if (!wide) {   // the columns from the bitmap, through the accumulators' memory so that they leave coalesced
+        sync();
+        ccol = reinterpret_cast<int *>(acc);
+        for (int w = tid; w < nw; w += NT) {
+            const uint2 x = word[w];
+            unsigned m = x.x;
+            int t = (int)x.y;
+            const int cb = c0 + (w << 5);
+            while (m) {
+                ccol[t++] = cb + __ffs(m) - 1;
+                m &= m - 1;
+            }
+        }
+        sync();
+    }
+    for (int t = tid; t < z; t += NT) colC[Rb + t] = ccol[t];
+}
+
+size_t sym_smem(int width) { return (size_t)std::min(width, SYM_BLKS) * (ROW_BLK / 8) + 4 * ((size_t)width + 1); }
+
+unsigned warps_grid(long long rows) { return (unsigned)std::min<long long>(std::max<long long>((rows + 7) / 8, 1), 152 * 32); }
+
+template <int NT>
+cudaError_t numeric_class(cudaStream_t s, const RowArgs &g, const int4 *items, long long n, int c,
+                          const long long *rowptrC, int *colC, double *valC, int *flags)
+{
+    if (n <= 0) return cudaSuccess;
+    k_row_numeric<NT><<<(unsigned)n, NT, class_smem(c) + row_steps(NT) * sizeof(Step), s>>>(g, items, rowptrC, colC, valC, flags);
+    ::tsg::count_launch();
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t rows_init_attributes()
+{
+    const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const int most = (int)sym_smem(ROW_MAX_BLKS);
+    cudaError_t e = cudaFuncSetAttribute(k_row_symbolic<256>, dyn, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_row_symbolic<64>, dyn, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_row_symbolic<1024>, dyn, most);
+    const int num = class_smem(ITEM_CLASSES - 1) + row_steps(NT_WIDE) * (int)sizeof(Step);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_row_numeric<32>, dyn, num);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_row_numeric<NT_WIDE>, dyn, num);
+    return e;
+}
+
+cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out)
+{
+    const long long rows = (g.m + step - 1) / step;
+    k_row_sample<<<(unsigned)((rows + 7) / 8), 256, 0, pool.stream>>>(g, step, out);
+    ::tsg::count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat)
+{
+    int2 *ext = pool.alloc_n<int2>(g.k);
+    if (!ext) return pool.err;
+    k_row_extents<<<(unsigned)((g.k + 255) / 256), 256, 0, pool.stream>>>(g.rpB, g.colB, g.k, ext);
+    k_row_products<<<warps_grid(g.m), 256, 0, pool.stream>>>(g, ext, prod, rng, heavy, stat);
+    ::tsg::count_launch();
+    ::tsg::count_launch();
+    pool.free(ext);
+    return cudaGetLastError();
+}
+
+cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut)
+{
+    k_row_cuts<<<(unsigned)((g.k + 7) / 8), 256, 0, pool.stream>>>(g.rpB, g.colB, g.k, g.nblk, cut);
+    ::tsg::count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const unsigned *nheavy,
+                         int width, int *rowcnt, int4 *items, unsigned cap, unsigned *nitems, cudaStream_t side,
+                         cudaEvent_t fork, cudaEvent_t join)
+{
+    cudaStream_t s = pool.stream;
+    const size_t sm = sym_smem(width);
+    HeavyRows h;
+    int total = 0;
+    for (int c = 0; c < HEAVY_CLASSES; ++c) total += h.n[c] = (int)nheavy[c];
+    cudaError_t e = cudaEventRecord(fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+    if (e != cudaSuccess) return e;
+    if (total > 0) {   // the heaviest first: the others run beside their tail
+        HeavyRows hl = h;
+        hl.list = heavy;
+        hl.m = g.m;
+        k_row_symbolic<1024><<<(unsigned)total, 1024, sm, side>>>(g, prod, ROW_HEAVY, INT_MAX, hl, width, rowcnt, items, cap, nitems);
+        ::tsg::count_launch();
+    }
+    k_row_symbolic<256><<<(unsigned)g.m, 256, sm, s>>>(g, prod, ROW_TINY, ROW_HEAVY, h, width, rowcnt, items, cap, nitems);
+    k_row_symbolic<64><<<(unsigned)g.m, 64, sm, side>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, nitems);
+    ::tsg::count_launch();
+    ::tsg::count_launch();
+    e = cudaGetLastError();
+    cudaError_t j = cudaEventRecord(join, side);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(s, join, 0);
+    return e == cudaSuccess ? j : e;
+}
+
+cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigned cap, const unsigned *n,
+                        const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
+                        cudaEvent_t fork, cudaEvent_t join)
+{
+    cudaStream_t s = pool.stream;
+    cudaError_t e = cudaEventRecord(fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+    // two streams, the longest chains first on each: a class's last items run
+    // beside the next ones
+    constexpr int order[ITEM_CLASSES] = {2, 1, 0, 3, 4, 5};
+    for (int q = 0; q < ITEM_CLASSES && e == cudaSuccess; ++q) {
+        const int c = order[q];
+        cudaStream_t on = q % 2 ? s : side;
+        const int4 *list = items + (long long)c * cap;
+        e = c < CLASS_WARP ? numeric_class<32>(on, g, list, n[c], c, rowptrC, colC, valC, flags)
+                           : numeric_class<NT_WIDE>(on, g, list, n[c], c, rowptrC, colC, valC, flags);
+    }
+    cudaError_t j = cudaEventRecord(join, side);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(s, join, 0);
+    return e == cudaSuccess ? j : e;
+}
+
+}  // namespace tsg

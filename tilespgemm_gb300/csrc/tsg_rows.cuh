@@ -1,0 +1,92 @@
+// tsg_rows.cuh -- the row path's sizes and entry points (tsg_rows.cu).
+#pragma once
+#include "tsg_internal.cuh"
+
+namespace tsg {
+
+constexpr int ROW_BLK_LOG = 10, ROW_BLK = 1 << ROW_BLK_LOG;   // columns of a block: a warp of bitmap words
+constexpr int ITEM_T = 1024;                  // an item closes once its row's entries pass a multiple of this
+constexpr int ITEM_CAP = ITEM_T + ROW_BLK;    // entries of an item at most (a block adds at most ROW_BLK)
+constexpr int ITEM_BLKS = 16;                 // blocks of an item at most
+constexpr int LIGHT_ROW = 4096, LIGHT_BLKS = 256;   // rows of so few entries: one item per so many blocks
+constexpr int SYM_BLKS = 256;                 // blocks of the symbolic bitmap at a time (32 KB)
+constexpr int ROW_MAX_BLKS = 4096;            // blocks of C's columns at most (4 M columns)
+constexpr int ROW_HEAVY = 1 << 15;            // rows of more products take a CTA of 1,024 threads
+constexpr int ROW_TINY = 2048;                // rows of so few products take a CTA of 64 threads
+constexpr int HEAVY_CLASSES = 4;              // ... listed by weight: the longest chains start first
+__host__ __device__ inline int heavy_class(long long p)
+{
+    return p > 32 * ROW_HEAVY ? 3 : p > 8 * ROW_HEAVY ? 2 : p > 3 * ROW_HEAVY ? 1 : 0;
+}
+constexpr int ROW_GROUP = 4;                  // steps whose entries are loaded together
+constexpr int NT_WIDE = 128;                  // threads of the items whose A entries bring many products each
+static_assert(ROW_BLK == 1024, "a block is 32 bitmap words");
+
+__host__ __device__ constexpr int row_steps(int nt) { return nt > 32 ? 128 : 32; }   // steps staged at a time
+
+// Classes of items: shared memory beside the staged steps, so that an SM holds
+// 21, 14 and 6 single-warp items (the first CLASS_WARP classes) or 5, 3 and
+// 2 items of NT_WIDE threads; the classes of heavy rows' items decide the
+// occupancy that hides their loads (one class of 20 KB in place of the first
+// two: R-MAT 2^18 A*A^T 52.3 against 45.3 ms).
+constexpr int ITEM_CLASSES = 6, CLASS_WARP = 3;
+__host__ __device__ constexpr int class_smem(int c)
+{
+    return c == 0 ? 9 << 10 : c == 1 ? 14 << 10 : c == 2 ? 34 << 10 : c == 3 ? 40 << 10 : c == 4 ? 72 << 10 : 112 << 10;
+}
+
+// Items whose blocks are half full or more keep an accumulator per column:
+// no bitmap pass over their products, no ranks.
+__host__ __device__ inline bool item_dense(int z, int nb) { return nb * ROW_BLK <= 2 * z; }
+__host__ __device__ inline int item_smem(int z, int nb)
+{
+    return item_dense(z, nb) ? nb * ROW_BLK * 9 : nb * (ROW_BLK / 4) + z * (nb > ITEM_BLKS ? 12 : 8);
+}
+// each: products of an A entry in the item, on average.  Above 32 a light
+// row is NT_WIDE threads' work (R-MAT 2^12 A*A^T 489 -> 438 us); below, a step
+// of NT_WIDE would idle most of them (31^3 27-point stencil, 27 each: 383 us
+// as a warp's, 711 as a CTA's).  A heavy row's items are a warp's in any case.
+__host__ __device__ inline int item_class(int z, int nb, float each, bool light)
+{
+    const int b = item_smem(z, nb);
+    if (b <= class_smem(2) && (each <= 32 || !light)) return b <= class_smem(0) ? 0 : b <= class_smem(1) ? 1 : 2;
+    return b <= class_smem(3) ? 3 : b <= class_smem(4) ? 4 : 5;
+}
+static_assert(LIGHT_BLKS * (ROW_BLK / 4) + LIGHT_ROW * 12 <= class_smem(5), "every light row's item fits the last class");
+static_assert(LIGHT_ROW * 2 * 9 <= class_smem(5) && ITEM_CAP * 2 * 9 <= class_smem(5), "dense items fit");
+static_assert(ITEM_BLKS * (ROW_BLK / 4) + ITEM_CAP * 12 <= class_smem(2), "every other item fits a warp's classes");
+
+struct RowArgs {
+    int m = 0, k = 0, n = 0, nblk = 0;
+    const long long *rpA = nullptr, *rpB = nullptr;
+    const int *colA = nullptr, *colB = nullptr;
+    const double *valA = nullptr, *valB = nullptr;
+    const int2 *rng = nullptr;                // each row of C: its blocks [x, y)
+    const int *cut = nullptr;                 // k * (nblk + 1); null when every row is one item
+};
+
+// What row_products finds (zeroed before).
+struct RowStat {
+    unsigned long long products, items;       // intermediate products; an upper bound of the items
+    unsigned heavy[HEAVY_CLASSES];
+    int width;                                // blocks of the widest row
+    int cuts;                                 // a row needs the cut table (more than one item or window)
+    int bad;                                  // a column of A outside B's rows
+    int pad;
+    unsigned nitems[ITEM_CLASSES];            // row_symbolic: items of each class
+};
+
+cudaError_t rows_init_attributes();
+// adds step * the products of every step-th row
+cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out);
+cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat);
+cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut);
+// items: ITEM_CLASSES lists of cap
+cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const unsigned *nheavy,
+                         int width, int *rowcnt, int4 *items, unsigned cap, unsigned *nitems, cudaStream_t side,
+                         cudaEvent_t fork, cudaEvent_t join);
+cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigned cap, const unsigned *n,
+                        const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
+                        cudaEvent_t fork, cudaEvent_t join);
+
+}  // namespace tsg
