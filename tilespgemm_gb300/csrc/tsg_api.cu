@@ -12,6 +12,7 @@
 #include "tsg_internal.cuh"
 #include "tsg_mtx.h"
 #include "tsg_numeric.cuh"
+#include "tsg_rows.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -42,8 +43,8 @@ cudaError_t aux_gather(Pool &pool, const int *perm, const double *src, double *d
 cudaError_t aux_nnzcub(Pool &pool, const long long *rpA, const int *colA, int m, const long long *rpB, int kB,
                        unsigned long long *out);
 cudaError_t aux_mask_popc(Pool &pool, const int *trp, int blkm, const uint16_t *mask, unsigned long long *out);
-cudaError_t aux_rows_increasing(Pool &pool, const long long *rp, const int *col, int m, long long nnz,
-                                unsigned long long *out);
+cudaError_t aux_rows_increasing(Pool &pool, const long long *rp, const int *col, int m, int n, long long nnz,
+                                unsigned long long *out, unsigned long long *runs);
 cudaError_t aux_copy_scalars(Pool &pool, const long long *a, long long *da, const int *b, long long *db,
                              const int *c, long long *dc);
 cudaError_t aux_rowptr_narrow(Pool &pool, const long long *in, int *out, long long n);
@@ -165,6 +166,7 @@ struct tsg_ctx {
     cudaStream_t copy = nullptr;
     cudaEvent_t cfork = nullptr, vals_ev = nullptr, cols_ev = nullptr, copy_done = nullptr;
     cudaEvent_t ext_ev = nullptr;            // tsg_stream_wait: the caller's stream's point to wait for
+    Arena arena;                             // tsg_spgemm's scratch, kept between calls
     std::vector<SmallShape> small_shapes;   // the last SMALL_SHAPES shapes, newest last
 };
 
@@ -312,6 +314,34 @@ struct DevCSR {
     long long *rp = nullptr;   // int64, clamped
     const int *col = nullptr;
     const double *val = nullptr;
+};
+
+// One tsg_spgemm call's use of its context's arena: empty at the start
+// (the call before is ahead of it on the context's stream), grown at the end
+// to what the call asked for.
+struct ArenaUse {
+    Arena &a;
+    Pool &pool;
+    ArenaUse(Arena &arena, Pool &p) : a(arena), pool(p) {
+        a.used = a.asked = 0;
+        if (a.want > a.cap) {
+            drop();
+            size_t bytes = a.want;
+            if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&a.base), bytes, p.pool, p.stream) == cudaSuccess) a.cap = bytes;
+            else { a.base = nullptr; cudaGetLastError(); }
+            a.want = 0;
+        }
+        pool.arena = &a;
+    }
+    void drop() {   // back to the pool, after the work that uses it
+        if (a.base) cudaFreeAsync(a.base, pool.stream);
+        a.base = nullptr;
+        a.cap = a.used = 0;
+    }
+    ~ArenaUse() {
+        if (a.asked > a.cap && a.asked <= ARENA_MAX) a.want = a.asked;
+        pool.arena = nullptr;
+    }
 };
 
 // Everything one call allocates from the pool; released together.
@@ -531,10 +561,30 @@ tsg_status stage_into_plan(tsg_ctx *ctx, Pool &pool, PlanData &P, const tsg_csr 
     return TSG_OK;
 }
 
+// Whether the row path (tsg_rows.cu) takes a product: `products` is the
+// sampled estimate, runs the operands' tile runs.
+// - Under 24 M products the tiled path's 25 launches and half-empty kernels
+//   cost more than its tiles save (31^3 27-point stencil, 19 M: 455 us tiled,
+//   383 by rows; R-MAT 2^12: 1,180 and 440); large ones only with fewer than
+//   1.5 entries a tile run (200,000 rows of 20 in a band of +-300, 1.25 a run:
+//   1,447 us tiled, 1,295 by rows; +-100, 1.84: 1,066 and 1,279).
+// - A row costs the row path a few microseconds of a CTA whatever it holds:
+//   rows of under 128 products go by tiles when there are many (96^3 7-point
+//   stencil, 48 a row: 2.0 ms tiled, 5.2 by rows).
+bool rows_pay(const PlanData &P, long long products, long long runsA, long long runsB)
+{
+    const bool full = products >= 128ll * P.m;
+    if (products <= 24000000) return full || P.m <= 65536;
+    return full && 2 * P.nnzA < 3 * runsA && 2 * P.nnzB < 3 * runsB;
+}
+
 // Symbolic phase: staging, A^T for A*A^T, tiles, step 1, step 2 (two host waits).
 // `keep` = the plan outlives the call (device operands are copied).
+// by_rows (optional): the caller can take the row path; set when the staged
+// operands qualify for it, and then nothing but the staging is done.
 tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const tsg_csr *A, const tsg_csr *B,
-                         PlanData &P, bool keep, bool want_cub, PhaseTimer &tm, bool reset_flags = true)
+                         PlanData &P, bool keep, bool want_cub, PhaseTimer &tm, bool reset_flags = true,
+                         bool *by_rows = nullptr)
 {
     const bool validate = ctx->opts.validate != 0;
     tsg_status r = check_op(op, A, B);
@@ -573,6 +623,33 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
         P.valA_buf = P.own<double>(pool, P.nnzA);
         if (!P.valA_buf) return fail(TSG_ERR_OOM, "device pool allocation failed");
     }
+    bool order_known = false;      // B's order is already counted
+    long long unsorted = 0;
+    if (by_rows) {
+        *by_rows = false;
+        const int nblk = ceil_div_i(P.n, ROW_BLK);
+        if (P.nnzA > 0 && P.nnzB > 0 && nblk <= ROW_MAX_BLKS) {
+            // tile runs of A and B, sampled products, and whether B's rows increase, decide
+            unsigned long long *rs = reinterpret_cast<unsigned long long *>(ctx->dstat);
+            if (op != TSG_OP_AA)
+                CUDA_OK(aux_rows_increasing(pool, P.rpA, P.colA, P.m, P.k, P.nnzA, rs + ST_NNZCUB, rs + ST_TILESA));
+            CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.n, P.nnzB, rs + ST_BUNSORTED, rs + ST_TILESB));
+            RowArgs g;
+            g.m = P.m; g.k = P.k; g.rpA = P.rpA; g.colA = P.colA; g.rpB = P.rpB;
+            CUDA_OK(row_sample(pool, g, P.m < 4096 ? 1 : 16, rs + ST_NNZC));
+            r = host_wait(ctx, &P.nsync);
+            if (r) return r;
+            const long long runsB = ctx->hstat[ST_TILESB], runsA = op == TSG_OP_AA ? runsB : ctx->hstat[ST_TILESA];
+            order_known = true;
+            unsorted = ctx->hstat[ST_BUNSORTED];
+            if (unsorted == 0 && rows_pay(P, ctx->hstat[ST_NNZC], runsA, runsB)) {
+                *by_rows = true;
+                CUDA_OK(cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_HFLAGS, ctx->stream));
+                return TSG_OK;
+            }
+            CUDA_OK(cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_HFLAGS, ctx->stream));
+        }
+    }
     DevCSR dA, dB;
     dA.m = P.m; dA.n = P.k; dA.nnz = P.nnzA; dA.rp = P.rpA; dA.col = P.colA;
     dB.m = P.k; dB.n = P.n; dB.nnz = P.nnzB; dB.rp = P.rpB; dB.col = P.colB;
@@ -610,7 +687,8 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
     {
         size_t free_b = 0, total_b = 0;
         const long long bytes = 4ll * wpr * P.blkm;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= (2ll << 30) && bytes <= (long long)(free_b / 8))
+        if (bytes <= (64ll << 20) ||      // not worth the query
+            (bytes <= (2ll << 30) && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= (long long)(free_b / 8)))
             wbm = sc.get<unsigned>(wpr * P.blkm);
         cudaGetLastError();
     }
@@ -620,7 +698,9 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
     CUDA_OK(aux_copy_scalars(pool, P.crp + P.blkm, ctx->dstat + ST_NUMBLKC, TA.trp + TA.blkm, ctx->dstat + ST_TILESA,
                              TB.trp + TB.blkm, ctx->dstat + ST_TILESB));
     CUDA_OK(aux_mask_popc(pool, TB.trp, TB.blkm, TB.mask, (unsigned long long *)(ctx->dstat + ST_POPCB)));
-    CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.nnzB, (unsigned long long *)(ctx->dstat + ST_BUNSORTED)));
+    if (!order_known)
+        CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.n, P.nnzB,
+                                    (unsigned long long *)(ctx->dstat + ST_BUNSORTED), nullptr));
     if (want_cub)
         CUDA_OK(aux_nnzcub(pool, P.rpA, P.colA, P.m, P.rpB, P.k, (unsigned long long *)(ctx->dstat + ST_NNZCUB)));
     r = host_wait(ctx, &P.nsync);
@@ -632,7 +712,7 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
     P.tilesA = ctx->hstat[ST_TILESA];
     P.tilesB = ctx->hstat[ST_TILESB];
     P.dupsafe = ctx->hstat[ST_POPCB] != P.nnzB;
-    P.b_increasing = ctx->hstat[ST_BUNSORTED] == 0;
+    P.b_increasing = (order_known ? unsorted : ctx->hstat[ST_BUNSORTED]) == 0;
     P.nnzcub = ctx->hstat[ST_NNZCUB];
     if (P.numblkC >= (1ll << 31)) return fail(TSG_ERR_NOT_SUPPORTED, "C has %lld tiles; the limit is 2^31-1", P.numblkC);
 
@@ -726,11 +806,11 @@ void fill_stats(const PlanData &P, tsg_stats *st)
 cudaError_t output_rowptr(tsg_ctx *ctx, Pool &pool, int m, int bits, const long long *rowptr, void *&rp_dev)
 {
     if (bits == 32) {
-        int *rp32 = pool.alloc_n<int>(m + 1);
+        int *rp32 = pool.out_n<int>(m + 1);
         rp_dev = rp32;
         return rp32 ? aux_rowptr_narrow(pool, rowptr, rp32, m + 1) : cudaErrorMemoryAllocation;
     }
-    long long *rp64 = pool.alloc_n<long long>(m + 1);
+    long long *rp64 = pool.out_n<long long>(m + 1);
     rp_dev = rp64;
     return rp64 ? cudaMemcpyAsync(rp64, rowptr, sizeof(long long) * (size_t)(m + 1), cudaMemcpyDeviceToDevice, ctx->stream)
                 : cudaErrorMemoryAllocation;
@@ -888,6 +968,70 @@ void phase_times(tsg_ctx *ctx, tsg_stats *st, const PhaseTimer &tm)
     st->ms_convert = a; st->ms_step1 = b; st->ms_step2 = c1; st->ms_step3 = d;
 }
 
+
+// ---- the row path ---------------------------------------------------------------
+
+// C = A*B row by row from the staged operands (tsg_rows.cu): its products
+// and items' bound (a host wait), the cut table, C's row counts and items, the
+// scan (a host wait for C's size), then the items.  taken = false: it has no
+// room for its tables or an operand is out of range, and the tiled path runs.
+tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double *&val, bool &taken)
+{
+    taken = false;
+    RowArgs g;
+    g.m = P.m; g.k = P.k; g.n = P.n; g.nblk = ceil_div_i(P.n, ROW_BLK);
+    g.rpA = P.rpA; g.rpB = P.rpB; g.colA = P.colA; g.colB = P.colB; g.valA = P.valA; g.valB = P.valB;
+    Scratch sc(pool);
+    static_assert(sizeof(RowStat) <= 8 * BS_SLOTS, "the row path's statistics fit the bins' slots");
+    RowStat *rs = reinterpret_cast<RowStat *>(ctx->dstat + ST_BINS), h;
+    int *prod = sc.get<int>(P.m), *heavy = sc.get<int>((long long)HEAVY_CLASSES * P.m), *rowcnt = sc.get<int>(P.m + 1);
+    int2 *rng = sc.get<int2>(P.m);
+    P.rowptrC = P.own<long long>(pool, P.m + 1);
+    if (!prod || !heavy || !rowcnt || !rng || !P.rowptrC) return fail(TSG_ERR_OOM, "device pool allocation failed (row path)");
+    g.rng = rng;
+    CUDA_OK(row_products(pool, g, prod, rng, heavy, rs));
+    tsg_status r = host_wait(ctx, &P.nsync);
+    if (r) return r;
+    memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
+    const long long cap = std::max<long long>((long long)h.items, 1);
+    if (h.bad || cap >= (1ll << 30)) return TSG_OK;
+    if (h.cuts) {   // the cut table: at most a sixteenth of the free device memory
+        const long long n = (long long)P.k * (g.nblk + 1);
+        size_t free_b = 0, total_b = 0;
+        if (4 * n > (64ll << 20) &&
+            (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 4 * n > (long long)(free_b / 16))) {
+            cudaGetLastError();
+            return TSG_OK;
+        }
+        int *cut = sc.get<int>(n);
+        if (!cut) return fail(TSG_ERR_OOM, "device pool allocation failed (cut table)");
+        CUDA_OK(row_cuts(pool, g, cut));
+        g.cut = cut;
+    }
+    int4 *items = sc.get<int4>(ITEM_CLASSES * cap);
+    if (!items) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's items)");
+    CUDA_OK(row_symbolic(pool, g, prod, heavy, h.heavy, h.width, rowcnt, items, (unsigned)cap, rs->nitems, ctx->side,
+                         ctx->fork, ctx->join));
+    CUDA_OK(scan_i32_to_i64(pool, rowcnt, P.rowptrC, P.m, ctx->dflags));
+    CUDA_OK(cudaMemcpyAsync(ctx->dstat + ST_NNZC, P.rowptrC + P.m, sizeof(long long), cudaMemcpyDeviceToDevice,
+                            ctx->stream));
+    r = host_wait(ctx, &P.nsync);
+    if (r) return r;
+    P.nnzC = ctx->hstat[ST_NNZC];
+    memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
+    for (unsigned n : h.nitems)
+        if (n > cap) return fail(TSG_ERR_CUDA, "internal: the row path's items outgrew their bound");
+    if (output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))
+        return fail(TSG_ERR_INT32_OVERFLOW, "C has %lld entries; int32 row pointers cannot hold them", P.nnzC);
+    col = pool.out_n<int>(P.nnzC);
+    val = pool.out_n<double>(P.nnzC);
+    if (!col || !val) return fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
+    P.wait_values(ctx->stream);
+    CUDA_OK(row_numeric(pool, g, items, (unsigned)cap, h.nitems, P.rowptrC, col, val, ctx->dflags, ctx->side,
+                        ctx->fork, ctx->join));
+    taken = true;
+    return TSG_OK;
+}
 
 // ---- the small-product path ---------------------------------------------------
 
@@ -1304,6 +1448,7 @@ tsg_status tsg_create(tsg_ctx **out, int device, const tsg_opts *opts)
     cudaError_t e = tiles_init_attributes();
     if (e == cudaSuccess) e = symbolic_init_attributes();
     if (e == cudaSuccess) e = numeric_init_attributes();
+    if (e == cudaSuccess) e = rows_init_attributes();
     if (e != cudaSuccess) return cleanup(fail(TSG_ERR_CUDA, "kernel attributes: %s", cudaGetErrorString(e)));
     noalloc_forget(device);   // tsg_tiles_to_csr_noalloc resolves its scratch address again
     *out = c;
@@ -1323,6 +1468,7 @@ tsg_status tsg_destroy(tsg_ctx *c)
     if (c->copy) { cudaStreamSynchronize(c->copy); cudaStreamDestroy(c->copy); }
     for (cudaEvent_t e : {c->cfork, c->vals_ev, c->cols_ev, c->copy_done, c->ext_ev}) if (e) cudaEventDestroy(e);
     for (auto &sh : c->small_shapes) if (sh.rowptr) cudaFreeAsync(sh.rowptr, c->stream);
+    if (c->arena.base) cudaFreeAsync(c->arena.base, c->stream);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->dstat) cudaFree(c->dstat);
     if (c->hstat) cudaFreeHost(c->hstat);
@@ -1373,6 +1519,7 @@ tsg_status tsg_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr *
         if (taken) return rs;
     }
     Pool pool{ctx->pool, ctx->stream};
+    ArenaUse arena(ctx->arena, pool);
     PlanData P;
     PhaseTimer tm(ctx, st && ctx->opts.phase_times);
     int *col = nullptr;
@@ -1381,12 +1528,29 @@ tsg_status tsg_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr *
     tsg_status r;
     {
         Scratch sc(pool);
-        r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, st != nullptr && ctx->opts.count_products, tm);
+        // a call without statistics (of tiles and bins) may go by rows
+        bool by_rows = false;
+        r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, st != nullptr && ctx->opts.count_products, tm, true,
+                          !st && ctx->opts.small_path ? &by_rows : nullptr);
+        if (!r && by_rows) {
+            bool taken = false;
+            r = rows_product(ctx, pool, P, col, val, taken);
+            if (!r && taken) {
+                r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st);   // frees col and val on failure
+                P.release(pool);
+                return r;
+            }
+            if (!r) {   // no room for its tables: the tiled path, from the start
+                P.release(pool);
+                P = PlanData();
+                r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, false, tm);
+            }
+        }
         if (!r && output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))   // before any work on C
             r = fail(TSG_ERR_INT32_OVERFLOW, "C has %lld entries; int32 row pointers cannot hold them", P.nnzC);
         if (!r) {
-            col = pool.alloc_n<int>(P.nnzC);
-            val = pool.alloc_n<double>(P.nnzC);
+            col = pool.out_n<int>(P.nnzC);
+            val = pool.out_n<double>(P.nnzC);
             if (!col || !val) r = fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
         }
         if (!r && early_out_pays(P, C)) r = early_out_begin(ctx, pool, P, col, val, eo);
@@ -1397,6 +1561,7 @@ tsg_status tsg_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr *
         early_out_abort(ctx, pool, eo);
         pool.free(col); pool.free(val);
         P.release(pool);
+        if (r == TSG_ERR_OOM) arena.drop();
         cudaStreamSynchronize(ctx->stream);
         cudaGetLastError();
         return r;

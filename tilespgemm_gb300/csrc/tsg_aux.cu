@@ -66,29 +66,39 @@ __global__ void k_mark_row_starts(const long long *__restrict__ rp, int m, unsig
     }
 }
 
-// pairs (q, q+1) inside one row with col[q] >= col[q+1]; each thread takes
-// DESC_PER consecutive pairs, so the warp's reduction is paid once per
-// DESC_PER entries (one per entry took 65 us on 23 M entries)
+// pairs (q, q+1) inside one row with col[q] >= col[q+1], and columns outside
+// [0, n); with RUNS also the tile runs (entries that start a row or lie in
+// another 16-column tile than the entry before).  Each thread takes DESC_PER
+// consecutive pairs, so the warp's reduction is paid once per DESC_PER
+// entries (one per entry took 65 us on 23 M entries)
 constexpr int DESC_PER = 8;
-__global__ void k_count_descents(const int *__restrict__ col, long long nnz, const unsigned *__restrict__ starts,
-                                 unsigned long long *out)
+template <bool RUNS>
+__global__ void k_count_descents(const int *__restrict__ col, long long nnz, int n, const unsigned *__restrict__ starts,
+                                 unsigned long long *out, unsigned long long *runs)
 {
-    unsigned long long cnt = 0;
+    unsigned cnt = 0, nr = 0;
     const long long stride = (long long)gridDim.x * blockDim.x * DESC_PER;
-    for (long long q0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * DESC_PER; q0 + 1 < nnz; q0 += stride) {
+    for (long long q0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * DESC_PER; q0 < nnz; q0 += stride) {
         int prev = col[q0];
+        if (q0 == 0 && (unsigned)prev >= (unsigned)n) ++cnt;
 #pragma unroll
         for (int j = 1; j <= DESC_PER; ++j) {
             const long long n1 = q0 + j;
             if (n1 < nnz) {
                 const int cur = col[n1];
-                if (!((starts[n1 >> 5] >> (n1 & 31)) & 1u) && prev >= cur) ++cnt;
+                const bool first = (starts[n1 >> 5] >> (n1 & 31)) & 1u;
+                if ((!first && prev >= cur) || (unsigned)cur >= (unsigned)n) ++cnt;
+                if (RUNS && (first || (prev >> 4) != (cur >> 4))) ++nr;
                 prev = cur;
             }
         }
     }
-    cnt = (unsigned long long)warp_sum_ll((long long)cnt);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(out, cnt);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(out, (unsigned long long)cnt);
+    if (RUNS) {
+        nr = __reduce_add_sync(0xffffffffu, nr);
+        if ((threadIdx.x & 31) == 0 && nr) atomicAdd(runs, (unsigned long long)nr);
+    }
 }
 
 __global__ void k_copy_scalars(const long long *a, long long *da, const int *b, long long *db, const int *c, long long *dc)
@@ -411,16 +421,21 @@ cudaError_t aux_nnzcub(Pool &pool, const long long *rpA, const int *colA, int m,
     return cudaGetLastError();
 }
 
-cudaError_t aux_rows_increasing(Pool &pool, const long long *rp, const int *col, int m, long long nnz,
-                                unsigned long long *out)
+cudaError_t aux_rows_increasing(Pool &pool, const long long *rp, const int *col, int m, int n, long long nnz,
+                                unsigned long long *out, unsigned long long *runs)
 {
-    if (m <= 0 || nnz <= 1) return cudaSuccess;
+    if (m <= 0 || nnz <= 0) return cudaSuccess;
     const long long words = (nnz + 31) / 32 + 1;
     unsigned *starts = pool.alloc_n<unsigned>(words);
     if (!starts) return pool.err;
     cudaError_t e = cudaMemsetAsync(starts, 0, sizeof(unsigned) * (size_t)words, pool.stream);
     if (e == cudaSuccess) { k_mark_row_starts<<<g256(m), 256, 0, pool.stream>>>(rp, m, starts); ::tsg::count_launch(); }
-    if (e == cudaSuccess) { k_count_descents<<<g256((nnz + DESC_PER - 1) / DESC_PER), 256, 0, pool.stream>>>(col, nnz, starts, out); ::tsg::count_launch(); }
+    if (e == cudaSuccess) {
+        const unsigned grid = g256((nnz + DESC_PER - 1) / DESC_PER);
+        if (runs) k_count_descents<true><<<grid, 256, 0, pool.stream>>>(col, nnz, n, starts, out, runs);
+        else k_count_descents<false><<<grid, 256, 0, pool.stream>>>(col, nnz, n, starts, out, nullptr);
+        ::tsg::count_launch();
+    }
     if (e == cudaSuccess) e = cudaGetLastError();
     pool.free(starts);
     return e;
