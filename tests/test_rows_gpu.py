@@ -125,3 +125,20 @@ def test_rows_bad_columns(rctx):
     with pytest.raises(_abi.TSGError):
         rctx.spgemm(A, CSR(B.m, B.n, B.rowptr, col, B.val), op=op)
     _check(rctx.spgemm(A, B, op=op), O.spgemm(A, B))
+
+
+@pytest.mark.parametrize("op", ["AA", "AAT", "AB"])
+def test_batched_rows(rctx, op):
+    """A batch by the row path (instances that start inside a block, widths
+    around one, a heavy row with several items): each equals its oracle."""
+    shapes = [(90, 90), (1040, 1040), (1, 1), (2100, 2100), (37, 37), (5000, 5000)]
+    if op != "AA":
+        shapes = [(m, n + 3 * i) for i, (m, n) in enumerate(shapes)]
+    As = [_rows(m, n, [min(n, 20), 3, min(n, 90)], 40 + i) for i, (m, n) in enumerate(shapes)]
+    As.append(_rows(12, 12 if op == "AA" else 300, [250, 5], 50))
+    Bs = None
+    if op == "AB":
+        Bs = [_rows(A.n, 700 + 2000 * i, [40, 0, 600], 60 + i) for i, A in enumerate(As)]
+    got = rctx.spgemm_batched(As, Bs, op=op)
+    for i, A in enumerate(As):
+        _check(got[i], O.spgemm(A, _b(A, Bs[i] if Bs else None, op)))

@@ -627,8 +627,7 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
     long long unsorted = 0;
     if (by_rows) {
         *by_rows = false;
-        const int nblk = ceil_div_i(P.n, ROW_BLK);
-        if (P.nnzA > 0 && P.nnzB > 0 && nblk <= ROW_MAX_BLKS) {
+        if (P.nnzA > 0 && P.nnzB > 0) {
             // tile runs of A and B, sampled products, and whether B's rows increase, decide
             unsigned long long *rs = reinterpret_cast<unsigned long long *>(ctx->dstat);
             if (op != TSG_OP_AA)
@@ -975,12 +974,21 @@ void phase_times(tsg_ctx *ctx, tsg_stats *st, const PhaseTimer &tm)
 // and items' bound (a host wait), the cut table, C's row counts and items, the
 // scan (a host wait for C's size), then the items.  taken = false: it has no
 // room for its tables or an operand is out of range, and the tiled path runs.
-tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double *&val, bool &taken)
+// batch (optional): the packed instances' layout.
+struct RowBatch {
+    const int *base = nullptr, *coloff = nullptr;   // device: RowArgs's
+    int width = 0;                                  // blocks of the widest instance
+};
+
+tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double *&val, bool &taken,
+                        const RowBatch *batch = nullptr)
 {
     taken = false;
     RowArgs g;
     g.m = P.m; g.k = P.k; g.n = P.n; g.nblk = ceil_div_i(P.n, ROW_BLK);
     g.rpA = P.rpA; g.rpB = P.rpB; g.colA = P.colA; g.colB = P.colB; g.valA = P.valA; g.valB = P.valB;
+    g.width = g.nblk;
+    if (batch) { g.base = batch->base; g.width = batch->width; g.coloff = batch->coloff; }
     Scratch sc(pool);
     static_assert(sizeof(RowStat) <= 8 * BS_SLOTS, "the row path's statistics fit the bins' slots");
     RowStat *rs = reinterpret_cast<RowStat *>(ctx->dstat + ST_BINS), h;
@@ -994,9 +1002,9 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     if (r) return r;
     memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
     const long long cap = std::max<long long>((long long)h.items, 1);
-    if (h.bad || cap >= (1ll << 30)) return TSG_OK;
+    if (h.bad || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS) return TSG_OK;
     if (h.cuts) {   // the cut table: at most a sixteenth of the free device memory
-        const long long n = (long long)P.k * (g.nblk + 1);
+        const long long n = (long long)P.k * (g.width + 1);
         size_t free_b = 0, total_b = 0;
         if (4 * n > (64ll << 20) &&
             (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 4 * n > (long long)(free_b / 16))) {
@@ -1009,6 +1017,11 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
         g.cut = cut;
     }
     int4 *items = sc.get<int4>(ITEM_CLASSES * cap);
+    // light rows go to CTAs from 32 products an A entry on where the chains of
+    // a small product decide (R-MAT 2^12 A*A^T: 430 us, 509 with 64; 31^3
+    // stencil, 27 each: 383 us by warps, 711 by CTAs), from 64 on where the
+    // SMs are full (512 mixed products: 30.7 ms with 64, 36.6 with 32, 39.1 with 200)
+    g.each = h.products > 24000000 ? 64.0f : 32.0f;
     if (!items) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's items)");
     CUDA_OK(row_symbolic(pool, g, prod, heavy, h.heavy, h.width, rowcnt, items, (unsigned)cap, rs->nitems, ctx->side,
                          ctx->fork, ctx->join));
@@ -1021,7 +1034,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
     for (unsigned n : h.nitems)
         if (n > cap) return fail(TSG_ERR_CUDA, "internal: the row path's items outgrew their bound");
-    if (output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))
+    if (!batch && output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))
         return fail(TSG_ERR_INT32_OVERFLOW, "C has %lld entries; int32 row pointers cannot hold them", P.nnzC);
     col = pool.out_n<int>(P.nnzC);
     val = pool.out_n<double>(P.nnzC);
@@ -2325,6 +2338,7 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         noff[i] = N; N += round16(ni);
     }
     Pool pool{ctx->pool, ctx->stream};
+    ArenaUse arena(ctx->arena, pool);
     PlanData P;
     PhaseTimer tm(ctx, st && ctx->opts.phase_times);
     int *col = nullptr;
@@ -2337,8 +2351,9 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         r = pack_operands(ctx, pool, sc, count, A, roff, op == TSG_OP_AAT ? koff : (op == TSG_OP_AA ? roff : koff),
                           M, op == TSG_OP_AA ? M : K, pA);
         if (!r && op == TSG_OP_AB) r = pack_operands(ctx, pool, sc, count, B, koff, noff, K, N, pB);
+        bool by_rows = false;
         if (!r) r = plan_symbolic(ctx, pool, sc, op, &pA, op == TSG_OP_AB ? &pB : nullptr, P, false, st != nullptr && ctx->opts.count_products, tm,
-                                  false);
+                                  false, !st && ctx->opts.small_path ? &by_rows : nullptr);
         // C's column offset of each packed tile-row's instance: the numeric
         // step writes C_i's columns already rebased
         long long rpn = 0;
@@ -2352,14 +2367,38 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         }
         int *d_trc = nullptr;
         if (!r) {
-            col = pool.alloc_n<int>(P.nnzC);
-            val = pool.alloc_n<double>(P.nnzC);
             d_trc = sc.get<int>((long long)trc.size());
-            if (!col || !val || !d_trc) r = fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
+            if (!d_trc) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch layout)");
         }
-        if (!r) {
-            CUDA_OK(cudaMemcpyAsync(d_trc, trc.data(), sizeof(int) * trc.size(), cudaMemcpyHostToDevice, ctx->stream));
-            r = plan_numeric(ctx, pool, P, P.valA, P.valB, col, val, d_trc);
+        if (!r) CUDA_OK(cudaMemcpyAsync(d_trc, trc.data(), sizeof(int) * trc.size(), cudaMemcpyHostToDevice, ctx->stream));
+        bool taken = false;
+        std::vector<int> base;
+        if (!r && by_rows) {
+            // per tile-row of B its instance's first block of C's columns
+            RowBatch rb;
+            base.assign((size_t)((op == TSG_OP_AA ? M : K) / TILE) + 1, 0);
+            for (int i = 0; i < count; ++i) {
+                const long long c0 = ud[i].coloff, b0 = op == TSG_OP_AA ? roff[i] : koff[i];
+                const int ni = op == TSG_OP_AB ? B[i].n : (op == TSG_OP_AA ? A[i].n : A[i].m);
+                for (long long t = b0 / TILE; t < (b0 + round16(A[i].n)) / TILE; ++t) base[(size_t)t] = (int)(c0 / ROW_BLK);
+                if (ni > 0) rb.width = std::max(rb.width, (int)((c0 + ni - 1) / ROW_BLK - c0 / ROW_BLK + 1));
+            }
+            int *d_base = sc.get<int>((long long)base.size());
+            if (!d_base) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch layout)");
+            if (!r) CUDA_OK(cudaMemcpyAsync(d_base, base.data(), sizeof(int) * base.size(), cudaMemcpyHostToDevice, ctx->stream));
+            rb.base = d_base; rb.coloff = d_trc;
+            if (!r) r = rows_product(ctx, pool, P, col, val, taken, &rb);
+            if (!r && !taken) {
+                P.release(pool);
+                P = PlanData();
+                r = plan_symbolic(ctx, pool, sc, op, &pA, op == TSG_OP_AB ? &pB : nullptr, P, false, false, tm);
+            }
+        }
+        if (!r && !taken) {
+            col = pool.out_n<int>(P.nnzC);
+            val = pool.out_n<double>(P.nnzC);
+            if (!col || !val) r = fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
+            if (!r) r = plan_numeric(ctx, pool, P, P.valA, P.valB, col, val, d_trc);
         }
         tm.mark();  // 4
         // unpack: per-instance row pointers, rebased
@@ -2369,7 +2408,7 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         void *rp_out = nullptr;
         long long *ebase = nullptr;
         if (!r) {
-            rp_out = pool.alloc((size_t)rpn * (bits == 64 ? 8 : 4));
+            rp_out = pool.out((size_t)rpn * (bits == 64 ? 8 : 4));
             ebase = sc.get<long long>(count);
             UnpackDesc *dud = sc.get<UnpackDesc>(count);
             if (!rp_out || !ebase || !dud) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch outputs)");

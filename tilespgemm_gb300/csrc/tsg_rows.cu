@@ -139,26 +139,24 @@ k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, in
     }
 }
 
-// Row k of the cut table (one warp each): cut[k][j] = B's first entry of row
-// k at column j * ROW_BLK or past it; j = 0..nblk.  Written coalesced, read
+// Row k of the cut table (one warp each): B's first entry of row k at or past
+// each of width + 1 blocks from the row's base on.  Written coalesced, read
 // back by k_row_numeric as two neighbouring ints per A entry and item.
 __global__ void __launch_bounds__(256)
-k_row_cuts(const long long *__restrict__ rpB, const int *__restrict__ colB, int kB, int nblk, int *__restrict__ cut)
+k_row_cuts(const long long *__restrict__ rpB, const int *__restrict__ colB, int kB, int width,
+           const int *__restrict__ base, int *__restrict__ cut)
 {
     const long long k = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (k >= kB) return;
-    const int b0 = (int)rpB[k], b1 = (int)rpB[k + 1];
-    int *row = cut + k * (nblk + 1);
-    for (int j = lane; j <= nblk; j += 32) {
+    const int b0 = (int)rpB[k], b1 = (int)rpB[k + 1], j0 = base ? base[k >> 4] : 0;
+    int *row = cut + k * (width + 1);
+    for (int j = lane; j <= width; j += 32) {
         int a = b0, b = b1;
-        if (j == nblk) a = b1;
-        else {
-            const int key = j << ROW_BLK_LOG;
-            while (a < b) {
-                const int md = (a + b) >> 1;
-                if (colB[md] < key) a = md + 1; else b = md;
-            }
+        const long long key = (long long)(j0 + j) << ROW_BLK_LOG;
+        while (a < b) {
+            const int md = (a + b) >> 1;
+            if (colB[md] < key) a = md + 1; else b = md;
         }
         row[j] = a;
     }
@@ -220,7 +218,7 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
                 const int k = g.colA[a];
                 if (nblk <= SYM_BLKS) { s = (int)g.rpB[k]; e = (int)g.rpB[k + 1]; }
                 else {
-                    const int *row = g.cut + (long long)k * (g.nblk + 1) + first + wb;
+                    const int *row = g.cuts(k, first + wb);
                     s = row[0];
                     e = row[nb];
                 }
@@ -295,7 +293,7 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
     auto close = [&](int j, int e, int pj, int pe, bool write) {   // blocks [pj, j), entries [pe, e) of the row
         const int z = e - pe, nb = j - pj;
         if (z <= 0) return;
-        const int c = item_class(z, nb, (float)p * (float)z / ((float)la * (float)cnt[nblk]), tclose > ITEM_T);
+        const int c = item_class(z, nb, tclose == ITEM_T || (float)p * (float)z <= g.each * (float)la * (float)cnt[nblk]);
         const unsigned i = atomicAdd(s_cls + c, 1u);
         if (write && i < cap) items[(unsigned long long)c * cap + i] = make_int4(r, first + pj, pe, (nb << 16) | z);
     };
@@ -338,7 +336,7 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
     if (cnt[nblk] <= LIGHT_ROW && nblk <= LIGHT_BLKS) {      // one item
         const int z = cnt[nblk];
         if (lane == 0 && z > 0) {
-            const int c = item_class(z, nblk, (float)p / (float)la, true);
+            const int c = item_class(z, nblk, (float)p <= g.each * (float)la);
             const unsigned i = atomicAdd(nitems + c, 1u);
             if (i < cap) items[(unsigned long long)c * cap + i] = make_int4(r, first, 0, (nblk << 16) | z);
         }
@@ -400,7 +398,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
             nav = g.valA[a + tid];
             if (whole) { ns = (int)g.rpB[nk]; ne = (int)g.rpB[nk + 1]; }
             else {
-                const int *row = g.cut + (long long)nk * (g.nblk + 1) + j0;
+                const int *row = g.cuts(nk, j0);
                 ns = row[0];
                 ne = row[nb];
             }
@@ -564,6 +562,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
         });
     };
     const long long Rb = rowptrC[r] + it.z;
+    const int shift = g.coloff ? g.coloff[r >> 4] : 0;
     if (dense) {
         values([&](int c, bool live) {
             const int o = live ? c - c0 : 0;
@@ -596,7 +595,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
             const int t = run + __popc(m & lanemask_lt());
             if (met && t < z) {
                 valC[Rb + t] = acc[w * 32 + lane];
-                colC[Rb + t] = c0 + w * 32 + lane;
+                colC[Rb + t] = c0 - shift + w * 32 + lane;
             }
             run += __popc(m);
         }
@@ -611,7 +610,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
     if (wide) {
         values([&](int c, bool live) {
             const int pos = rank(c);
-            if (live) ccol[pos] = c;
+            if (live) ccol[pos] = c - shift;
             return pos;
         });
     } else {
@@ -625,7 +624,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
             const uint2 x = word[w];
             unsigned m = x.x;
             int t = (int)x.y;
-            const int cb = c0 + (w << 5);
+            const int cb = c0 - shift + (w << 5);
             while (m) {
                 ccol[t++] = cb + __ffs(m) - 1;
                 m &= m - 1;
@@ -687,7 +686,7 @@ cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int
 
 cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut)
 {
-    k_row_cuts<<<(unsigned)((g.k + 7) / 8), 256, 0, pool.stream>>>(g.rpB, g.colB, g.k, g.nblk, cut);
+    k_row_cuts<<<(unsigned)((g.k + 7) / 8), 256, 0, pool.stream>>>(g.rpB, g.colB, g.k, g.width, g.base, cut);
     ::tsg::count_launch();
     return cudaGetLastError();
 }
@@ -730,7 +729,7 @@ cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigne
     if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
     // two streams, the longest chains first on each: a class's last items run
     // beside the next ones
-    constexpr int order[ITEM_CLASSES] = {2, 1, 0, 3, 4, 5};
+    constexpr int order[ITEM_CLASSES] = {3, 2, 1, 0, 4, 5, 6};
     for (int q = 0; q < ITEM_CLASSES && e == cudaSuccess; ++q) {
         const int c = order[q];
         cudaStream_t on = q % 2 ? s : side;

@@ -10,7 +10,7 @@ constexpr int ITEM_CAP = ITEM_T + ROW_BLK;    // entries of an item at most (a b
 constexpr int ITEM_BLKS = 16;                 // blocks of an item at most
 constexpr int LIGHT_ROW = 4096, LIGHT_BLKS = 256;   // rows of so few entries: one item per so many blocks
 constexpr int SYM_BLKS = 256;                 // blocks of the symbolic bitmap at a time (32 KB)
-constexpr int ROW_MAX_BLKS = 4096;            // blocks of C's columns at most (4 M columns)
+constexpr int ROW_MAX_BLKS = 4096;            // blocks of a row's columns at most (4 M columns)
 constexpr int ROW_HEAVY = 1 << 15;            // rows of more products take a CTA of 1,024 threads
 constexpr int ROW_TINY = 2048;                // rows of so few products take a CTA of 64 threads
 constexpr int HEAVY_CLASSES = 4;              // ... listed by weight: the longest chains start first
@@ -25,14 +25,13 @@ static_assert(ROW_BLK == 1024, "a block is 32 bitmap words");
 __host__ __device__ constexpr int row_steps(int nt) { return nt > 32 ? 128 : 32; }   // steps staged at a time
 
 // Classes of items: shared memory beside the staged steps, so that an SM holds
-// 21, 14 and 6 single-warp items (the first CLASS_WARP classes) or 5, 3 and
-// 2 items of NT_WIDE threads; the classes of heavy rows' items decide the
-// occupancy that hides their loads (one class of 20 KB in place of the first
-// two: R-MAT 2^18 A*A^T 52.3 against 45.3 ms).
-constexpr int ITEM_CLASSES = 6, CLASS_WARP = 3;
+// 21, 14, 10 and 6 single-warp items (the first CLASS_WARP classes) or 5, 3
+// and 2 items of NT_WIDE threads; the occupancy hides their loads (one class
+// of 20 KB in place of the first two: R-MAT 2^18 A*A^T 52.3 against 45.3 ms).
+constexpr int ITEM_CLASSES = 7, CLASS_WARP = 4;
 __host__ __device__ constexpr int class_smem(int c)
 {
-    return c == 0 ? 9 << 10 : c == 1 ? 14 << 10 : c == 2 ? 34 << 10 : c == 3 ? 40 << 10 : c == 4 ? 72 << 10 : 112 << 10;
+    return c == 0 ? 9 << 10 : c == 1 ? 14 << 10 : c == 2 ? 20 << 10 : c == 3 ? 34 << 10 : c == 4 ? 40 << 10 : c == 5 ? 72 << 10 : 112 << 10;
 }
 
 // Items whose blocks are half full or more keep an accumulator per column:
@@ -42,27 +41,36 @@ __host__ __device__ inline int item_smem(int z, int nb)
 {
     return item_dense(z, nb) ? nb * ROW_BLK * 9 : nb * (ROW_BLK / 4) + z * (nb > ITEM_BLKS ? 12 : 8);
 }
-// each: products of an A entry in the item, on average.  Above 32 a light
-// row is NT_WIDE threads' work (R-MAT 2^12 A*A^T 489 -> 438 us); below, a step
-// of NT_WIDE would idle most of them (31^3 27-point stencil, 27 each: 383 us
-// as a warp's, 711 as a CTA's).  A heavy row's items are a warp's in any case.
-__host__ __device__ inline int item_class(int z, int nb, float each, bool light)
+// warp: the item is one warp's where it fits.  A heavy row's always is; a
+// light row's while an A entry brings few products (RowArgs::each), for a
+// step of NT_WIDE would idle most of its threads.
+__host__ __device__ inline int item_class(int z, int nb, bool warp)
 {
     const int b = item_smem(z, nb);
-    if (b <= class_smem(2) && (each <= 32 || !light)) return b <= class_smem(0) ? 0 : b <= class_smem(1) ? 1 : 2;
-    return b <= class_smem(3) ? 3 : b <= class_smem(4) ? 4 : 5;
+    if (warp && b <= class_smem(3)) return b <= class_smem(0) ? 0 : b <= class_smem(1) ? 1 : b <= class_smem(2) ? 2 : 3;
+    return b <= class_smem(4) ? 4 : b <= class_smem(5) ? 5 : 6;
 }
-static_assert(LIGHT_BLKS * (ROW_BLK / 4) + LIGHT_ROW * 12 <= class_smem(5), "every light row's item fits the last class");
-static_assert(LIGHT_ROW * 2 * 9 <= class_smem(5) && ITEM_CAP * 2 * 9 <= class_smem(5), "dense items fit");
-static_assert(ITEM_BLKS * (ROW_BLK / 4) + ITEM_CAP * 12 <= class_smem(2), "every other item fits a warp's classes");
+static_assert(LIGHT_BLKS * (ROW_BLK / 4) + LIGHT_ROW * 12 <= class_smem(6), "every light row's item fits the last class");
+static_assert(LIGHT_ROW * 2 * 9 <= class_smem(6) && ITEM_CAP * 2 * 9 <= class_smem(6), "dense items fit");
+static_assert(ITEM_BLKS * (ROW_BLK / 4) + ITEM_CAP * 12 <= class_smem(3), "every other item fits a warp's classes");
 
 struct RowArgs {
     int m = 0, k = 0, n = 0, nblk = 0;
     const long long *rpA = nullptr, *rpB = nullptr;
     const int *colA = nullptr, *colB = nullptr;
     const double *valA = nullptr, *valB = nullptr;
+    float each = 32;                          // light rows: products of an A entry from which an item is a CTA's
     const int2 *rng = nullptr;                // each row of C: its blocks [x, y)
-    const int *cut = nullptr;                 // k * (nblk + 1); null when every row is one item
+    // The cut table, k rows of width + 1 blocks; null when every row is one
+    // item.  base (optional, batches): per 16 rows of B the block a table row
+    // starts at, so that it is as wide as an instance and not as the batch.
+    const int *cut = nullptr;
+    const int *base = nullptr;
+    int width = 0;
+    const int *coloff = nullptr;              // batches: per 16 rows of C, subtracted from its columns
+    __device__ __forceinline__ const int *cuts(int k, int j) const {   // B row k's, from block j on
+        return cut + (long long)k * (width + 1) + (j - (base ? base[k >> 4] : 0));
+    }
 };
 
 // What row_products finds (zeroed before).
