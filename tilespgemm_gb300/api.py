@@ -65,28 +65,29 @@ class CSR:
         return CSR(self.m, self.n, torch.as_tensor(np.asarray(self.rowptr)).to(dev),
                    torch.as_tensor(np.asarray(self.col)).to(dev), torch.as_tensor(np.asarray(self.val)).to(dev))
 
-    def _tsg(self, ctx_handle=None) -> tuple[_abi.tsg_csr, list]:
+    def _tsg(self, ctx_handle=None, synced: bool = False) -> tuple[_abi.tsg_csr, list]:
         """tsg_csr view of this matrix plus the objects that must stay alive.
         Device tensors: the context's stream (ctx_handle) is ordered after
         torch's current stream without blocking; without a context the host
-        waits for torch's stream."""
+        waits for torch's stream (synced: it has already)."""
         s = _abi.tsg_csr()
         s.m, s.n = int(self.m), int(self.n)
         keep: list = []
         if self.on_device:
             import torch
             rp, col, val = self.rowptr, self.col, self.val
-            if rp.dtype not in (torch.int32, torch.int64) or col.dtype != torch.int32 or val.dtype != torch.float64:
+            wide = rp.dtype == torch.int64
+            if not (wide or rp.dtype == torch.int32) or col.dtype != torch.int32 or val.dtype != torch.float64:
                 raise TypeError("device CSR needs int32/int64 row pointers, int32 columns, float64 values")
             rp, col, val = rp.contiguous(), col.contiguous(), val.contiguous()
             keep += [rp, col, val]
-            s.rowptr_bits = 64 if rp.dtype == torch.int64 else 32
+            s.rowptr_bits = 64 if wide else 32
             s.where = _abi.MEM_DEVICE
             s.row_ptr, s.col, s.val = rp.data_ptr(), col.data_ptr(), val.data_ptr()
-            s.nnz = int(col.numel())
+            s.nnz = col.numel()
             if ctx_handle:
                 check(lib().tsg_stream_wait(ctx_handle, torch.cuda.current_stream(rp.device).cuda_stream))
-            else:
+            elif not synced:
                 torch.cuda.current_stream(rp.device).synchronize()
         else:
             rp = np.asarray(self.rowptr)
@@ -411,14 +412,14 @@ class Context:
         a = (_abi.tsg_csr * max(n, 1))()
         keep: list = []
         for i, A in enumerate(As):
-            s_, k_ = A._tsg()
+            s_, k_ = A._tsg(synced=i > 0)
             a[i] = s_
             keep.append(k_)
         b_ptr = None
         if Bs is not None:
             b = (_abi.tsg_csr * max(n, 1))()
             for i, B in enumerate(Bs):
-                s_, k_ = B._tsg()
+                s_, k_ = B._tsg(synced=n > 0)
                 b[i] = s_
                 keep.append(k_)
             b_ptr = b
@@ -427,11 +428,7 @@ class Context:
         st = _abi.tsg_stats() if stats else None
         check(lib().tsg_spgemm_batched(self.handle, _OPS[op], n, a, b_ptr, c, C.byref(st) if st is not None else None))
         del keep
-        outs = []
-        for i in range(n):
-            cs = _abi.tsg_csr()
-            C.memmove(C.byref(cs), C.byref(c[i]), C.sizeof(_abi.tsg_csr))
-            outs.append(OwnedCSR(self, cs))
+        outs = [OwnedCSR(self, c[i]) for i in range(n)]
         return outs, (st.as_dict() if st is not None else None)
 
     def spgemm_batched(self, As: list, Bs: list | None = None, op: str = "AA") -> list:

@@ -179,6 +179,7 @@ enum StatSlot {
     ST_BUNSORTED = 36,           // B rows whose columns are not strictly increasing
     ST_SMALL = 37,               // small-product path: rows over its limit, products, a row past one round (3 slots)
     ST_HFLAGS = 40,              // device: the flags (FLAG_COUNT ints); host: their mirror as int64
+    ST_REPORT = 48,              // device: the small path's SmallReport; host: what it reports (2 + FLAG_COUNT slots)
     ST_SLOTS = 64
 };
 
@@ -429,7 +430,8 @@ tsg_status host_wait(tsg_ctx *ctx, int *nsync)
     // the statistics and, behind them, the flags: one copy
     CUDA_OK(cudaMemcpyAsync(ctx->hstat, ctx->dstat, sizeof(long long) * ST_HFLAGS + sizeof(int) * FLAG_COUNT,
                             cudaMemcpyDeviceToHost, ctx->stream));
-    static_assert(FLAG_COUNT <= ST_SLOTS - ST_HFLAGS, "flag mirror");
+    static_assert(FLAG_COUNT <= ST_REPORT - ST_HFLAGS, "flag mirror");
+    static_assert(sizeof(SmallReport) <= 8 * (ST_SLOTS - ST_REPORT) && 2 + FLAG_COUNT <= ST_SLOTS - ST_REPORT, "report");
     static_assert(ST_BINS + BS_SLOTS <= ST_BUNSORTED && ST_BUNSORTED < ST_SMALL && ST_SMALL + 3 <= ST_HFLAGS,
                   "statistics slots");
     int hflags[FLAG_COUNT];
@@ -1172,7 +1174,9 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
     };
     const bool validate = ctx->opts.validate != 0;
     unsigned long long *sstat = reinterpret_cast<unsigned long long *>(ctx->dstat + ST_SMALL);
-    cudaError_t e = cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_SLOTS, ctx->stream);   // flags too
+    cudaError_t e = cudaSuccess;
+    const bool one = seen && seen->rowptr && seen->one_round && A->m > 0;   // one launch, one wait
+    if (!one) e = cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_REPORT, ctx->stream);   // flags too
     if (e != cudaSuccess) return cuda_fail(e);
     P.op = op; P.m = A->m; P.k = A->n; P.nnzA = A->nnz;
     P.n = Bm->n; P.nnzB = Bm->nnz;
@@ -1184,7 +1188,7 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
     // buffers of `cap` entries, the fill at `rowptr` (kept: rows counted
     // against it), the caller's row pointer for device output, the wait
     auto fill = [&](const SmallOperands &so, const long long *rowptr, long long cap, bool kept,
-                    bool one_round) -> tsg_status {
+                    bool one_launch) -> tsg_status {
         if (dev_out) {
             auto a256 = [](long long x) { return (size_t)((x + 255) & ~255ll); };
             const size_t oc = a256(4 * std::max(cap, 1ll)), ov = a256(8 * std::max(cap, 1ll));
@@ -1201,8 +1205,20 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
         if (!col || !val) return fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", cap);
         P.wait_values(ctx->stream);
         // the fill writes the caller's row pointer too (device output)
-        cudaError_t fe = small_fill(pool, so, rowptr, cap, col, val, ctx->dflags, kept ? sstat : nullptr,
-                                    dev_out ? rp_dev : nullptr, bits, one_round);
+        void *rp = dev_out ? rp_dev : nullptr;
+        if (one_launch) {
+            long long *rep = ctx->hstat + ST_REPORT;
+            cudaError_t fe = small_fill_one(pool, so, rowptr, cap, col, val,
+                                            reinterpret_cast<SmallReport *>(ctx->dstat + ST_REPORT), rep, rp, bits);
+            if (fe == cudaSuccess) fe = cudaStreamSynchronize(ctx->stream);
+            if (fe != cudaSuccess) return fail(cuda_status(fe), "small path: %s", cudaGetErrorString(fe));
+            ++P.nsync;
+            ctx->hstat[ST_SMALL] = rep[0];
+            ctx->hstat[ST_SMALL + 1] = rep[1];
+            for (int f = 0; f < FLAG_COUNT; ++f) ctx->hstat[ST_HFLAGS + f] = rep[2 + f];
+            return read_flags(ctx);
+        }
+        cudaError_t fe = small_fill(pool, so, rowptr, cap, col, val, ctx->dflags, kept ? sstat : nullptr, rp, bits);
         if (fe != cudaSuccess) return fail(cuda_status(fe), "small path: %s", cudaGetErrorString(fe));
         return host_wait(ctx, &P.nsync);
     };
@@ -1215,7 +1231,7 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
         r = small_raw_operands(ctx, pool, P, op == TSG_OP_AA, A, Bm, ro);
         if (r) return give_up(r);
         ro.check = validate;
-        r = fill(ro, seen->rowptr, seen->nnzc, true, seen->one_round);
+        r = fill(ro, seen->rowptr, seen->nnzc, true, one);
         if (r) return give_up(r);
         if (ctx->hstat[ST_SMALL] == 0) {
             rowptr = seen->rowptr;
@@ -1223,7 +1239,7 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
         } else {   // a row differs from the kept pointer: the count pass decides
             drop_cv();
             P.release(pool);
-            e = cudaMemsetAsync(ctx->dstat + ST_SMALL, 0, 3 * sizeof(long long), ctx->stream);
+            e = cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_REPORT, ctx->stream);
             if (e != cudaSuccess) return cuda_fail(e);
         }
     }
@@ -1500,8 +1516,9 @@ tsg_status tsg_csr_free(tsg_ctx *ctx, tsg_csr *M)
         if (o->where == TSG_MEM_DEVICE) {
             if (c) {
                 cudaSetDevice(c->device);
+                // in stream order: the pool hands the memory on behind the
+                // work that is ahead on the context's stream
                 for (auto &b : o->blocks) cudaFreeAsync(b.first, c->stream);
-                cudaStreamSynchronize(c->stream);
             }
         } else if (o->where == TSG_MEM_HOST) {
             for (auto &b : o->blocks) pinned_put(c, b.first, b.second);   // kept, or freed past the cap
@@ -1844,7 +1861,7 @@ tsg_status tsg_load_mtx_device(tsg_ctx *ctx, const char *path, tsg_csr *A, int32
     const long long M = h.M, N = h.N, NZ = h.NZ;
     const char *data = text.data() + h.data;
     const long long nb = (long long)(text.size() - h.data);
-    cudaError_t e = cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_SLOTS, ctx->stream);   // flags too
+    cudaError_t e = cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_REPORT, ctx->stream);   // flags too
     char *dtext = static_cast<char *>(dalloc((size_t)((nb + 15) & ~15ll)));
     if (!dtext) return cuda_fail(cudaErrorMemoryAllocation);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dtext, data, (size_t)nb, cudaMemcpyHostToDevice, ctx->stream);
@@ -2033,7 +2050,7 @@ struct TilesOwner {
 
 void reset_dev_state(tsg_ctx *ctx)
 {
-    cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_SLOTS, ctx->stream);   // the flags inside it too
+    cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_REPORT, ctx->stream);   // the flags inside it too
 }
 
 __global__ void k_widen_i32(const int *in, long long *out, long long n)

@@ -226,8 +226,6 @@ struct RowPtr {
 // with `kept` non-null rowptrC is a row pointer kept from an earlier call:
 // rows that do not match it add 1 to kept[0] (products to kept[1]);
 // rp_out (optional) gets rowptrC as the caller's int32 or int64 row pointer;
-// one_round (with `kept`): a variant without shared memory for shapes
-// whose rows all fit one round (a row that does not counts in kept[0]).
 // ka = A's columns (= B's rows), nb = B's columns.
 constexpr int SMALL_MAX_PRODUCTS = 128;
 // The operands' row pointers are clamped into [0, nnz] where they are
@@ -244,8 +242,18 @@ struct SmallOperands {
 };
 cudaError_t small_count(Pool &pool, const SmallOperands &o, int *rowcnt, unsigned long long *stat);
 cudaError_t small_fill(Pool &pool, const SmallOperands &o, const long long *rowptrC, long long cap, int *colC,
-                       double *valC, int *flags, unsigned long long *kept = nullptr, void *rp_out = nullptr,
-                       int rp_bits = 32, bool one_round = false);
+                       double *valC, int *flags, unsigned long long *kept, void *rp_out, int rp_bits);
+// The kept fill for shapes whose rows all fit one round: the counts and flags
+// of the call go to `host` (pinned: kept[0], kept[1], the flags) with the
+// kernel's last CTA, which leaves *rep cleared: a call is one launch and one
+// wait, without the copies before and after it.
+struct SmallReport {
+    unsigned long long kept[2];
+    int flags[FLAG_COUNT];
+    unsigned done, pad;
+};
+cudaError_t small_fill_one(Pool &pool, const SmallOperands &o, const long long *rowptrC, long long cap, int *colC,
+                           double *valC, SmallReport *rep, long long *host, void *rp_out, int rp_bits);
 
 // One instance of a batched product, as the pack/unpack kernels see it.
 struct PackDesc {

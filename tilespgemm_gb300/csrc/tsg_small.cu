@@ -120,13 +120,18 @@ __device__ __forceinline__ int owner_lane(int off, int f)
 template <typename K>
 __device__ __forceinline__ K warp_sort_up(K key, int lane)
 {
+    // the lanes that sort downwards in a phase hold their keys complemented,
+    // so that a stage keeps the smaller or the larger by one bit of the lane
+    K flip = 0;
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1) {
+        const K down = (lane & k) && k < 32 ? ~(K)0 : (K)0;
+        key ^= flip ^ down;
+        flip = down;
 #pragma unroll
         for (int j = k >> 1; j > 0; j >>= 1) {
             const K other = __shfl_xor_sync(0xffffffffu, key, j);
-            const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
-            key = keep_min ? (other < key ? other : key) : (other > key ? other : key);
+            key = (lane & j) ? max(key, other) : min(key, other);
         }
     }
     return key;
@@ -217,28 +222,29 @@ k_small_count(SmallOperands o, int *rowcnt, unsigned long long *stat)
     }
 }
 
-// ONE: every row is expected to fit one round (a kept shape whose rows all
-// did): no hash tables, so no shared memory and more warps per SM; a row
-// that does not fit is reported through `kept` like a changed row.
-template <bool ONE>
-__global__ void __launch_bounds__(SH_WARPS * 32, ONE ? 6 : 1)
+// B's row pointer and columns, checked across the whole grid (A*B; with A*A
+// the rows' own checks cover them)
+__device__ __forceinline__ void check_b(const SmallOperands &o, int *flags)
+{
+    if (!o.check || o.b_is_a) return;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    bool bad = false;
+    for (long long i = t0; i <= o.kb; i += stride) {
+        const long long v = o.rpB[i];
+        bad |= v < 0 || v > o.nnzB || (i == 0 && v != 0) || (i == o.kb && v != o.nnzB) || (i < o.kb && o.rpB[i + 1] < v);
+    }
+    for (long long q = t0; q < o.nnzB; q += stride) bad |= (unsigned)o.colB[q] >= (unsigned)o.nb;
+    if (bad) set_flag(flags, FLAG_BAD_INPUT);
+}
+
+__global__ void __launch_bounds__(SH_WARPS * 32)
 k_small_fill(SmallOperands o, const long long *__restrict__ rowptrC, long long cap, int *colC, double *valC,
              int *flags, unsigned long long *kept, void *rp_out, int rp_bits)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * SH_WARPS + warp;
-    if (o.check && !o.b_is_a) {
-        // B's row pointer and columns, checked across the whole grid
-        const long long stride = (long long)gridDim.x * blockDim.x;
-        const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-        bool bad = false;
-        for (long long i = t0; i <= o.kb; i += stride) {
-            const long long v = o.rpB[i];
-            bad |= v < 0 || v > o.nnzB || (i == 0 && v != 0) || (i == o.kb && v != o.nnzB) || (i < o.kb && o.rpB[i + 1] < v);
-        }
-        for (long long q = t0; q < o.nnzB; q += stride) bad |= (unsigned)o.colB[q] >= (unsigned)o.nb;
-        if (bad) set_flag(flags, FLAG_BAD_INPUT);
-    }
+    check_b(o, flags);
     const int m = o.m;
     if (r >= m) return;
     const int *__restrict__ colB = o.colB;
@@ -321,10 +327,6 @@ k_small_fill(SmallOperands o, const long long *__restrict__ rowptrC, long long c
             return;
         }
     }
-    if constexpr (ONE) {
-        if (lane == 0) atomicAdd(kept, 1ull);   // not one round: the caller counts again
-        return;
-    } else {
     __shared__ int s_key[SH_WARPS][SH_CAP];
     __shared__ double s_val[SH_WARPS][SH_CAP];
     __shared__ int s_ck[SH_WARPS][SMALL_MAX_PRODUCTS];
@@ -407,6 +409,195 @@ k_small_fill(SmallOperands o, const long long *__restrict__ rowptrC, long long c
         colC[Rb + rank] = c;
         valC[Rb + rank] = cv[p];
     }
+}
+
+// The fill at a kept row pointer for shapes whose rows all fit one round (at
+// most 32 products from at most 32 A entries): a warp takes ONE_ROWS rows.
+//   1. the rows' A entries side by side, one a lane (rows follow one another in
+//      A), their B rows' places staged;
+//   2. per row, lane f holds product f; the keys (column, f) sorted across
+//      the warp put a column's products side by side in product order;
+//   3. the rows' entries of C, one a lane: its products applied in order.
+// A row that does not fit, or whose entries differ from the kept count, is
+// reported through `kept`; its C is not used then.
+// Bound by issue and by the FP64 pipe (a DFMA warp instruction holds it 20
+// clocks whatever its lanes): a row of its own a warp issued one DFMA per
+// product of its longest column, 5 on a 5-point Laplacian squared, 4 rows
+// together 2.5 a row, and the sorted products needed 12 shuffles each.
+// 256 x 256 Laplacian, A*A: 48 -> 33 us, 490 -> 315 instructions a row.
+constexpr int ONE_WARPS = 4;
+
+struct __align__(16) OneShare {   // an A entry's B row: entry f + delta for the group's product f
+    int delta, pad;
+    double a;
+};
+
+template <int ONE_ROWS>
+struct OneWarp {
+    double2 ab[ONE_ROWS * 32];         // products: A's and B's value
+    OneShare share[32];
+    uint2 out[ONE_ROWS * 32];          // entries of C: column, first sorted product | products << 8
+    unsigned char src[ONE_ROWS * 32];  // sorted products' places in ab
+};
+
+template <int ONE_ROWS, typename K>
+__global__ void __launch_bounds__(ONE_WARPS * 32)
+k_small_fill_one(SmallOperands o, const long long *__restrict__ rowptrC, long long cap, int *__restrict__ colC,
+                 double *__restrict__ valC, SmallReport *rep, long long *host, void *rp_out, int rp_bits)
+{
+    __shared__ OneWarp<ONE_ROWS> s_w[ONE_WARPS];
+    int *flags = rep->flags;
+    unsigned long long *kept = rep->kept;
+    __shared__ unsigned s_prod[ONE_WARPS];
+    constexpr unsigned FULL = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    check_b(o, flags);
+    OneWarp<ONE_ROWS> &w = s_w[warp];
+    const int m = o.m, nb = o.nb;
+    const int r0 = (blockIdx.x * ONE_WARPS + warp) * ONE_ROWS, nr = max(0, min(ONE_ROWS, m - r0));
+    unsigned products = 0;
+    if (nr > 0 && rowptrC[m] <= cap) {
+        // lane i: row r0 + i's span in A and C, and the caller's row pointer
+        int a0 = 0, a1 = 0, nc = 0;
+        long long Rb = 0;
+        if (lane < nr) {
+            const int r = r0 + lane;
+            long long s, e;
+            row_span(o.rpA, r, m, o.nnzA, o.check, 0, flags, s, e);
+            a0 = (int)s;
+            a1 = (int)e;
+            Rb = rowptrC[r];
+            const long long Re = rowptrC[r + 1];
+            nc = (int)(Re - Rb);
+            if (rp_out) {
+                if (rp_bits == 64) {
+                    static_cast<long long *>(rp_out)[r] = Rb;
+                    if (r == m - 1) static_cast<long long *>(rp_out)[m] = Re;
+                } else {
+                    static_cast<int *>(rp_out)[r] = (int)Rb;
+                    if (r == m - 1) static_cast<int *>(rp_out)[m] = (int)Re;
+                }
+            }
+        }
+        Rb = __shfl_sync(FULL, Rb, 0);
+        unsigned bad = 0;
+        int nout = 0;
+        for (int g0 = 0; g0 < nr;) {
+            // rows [g0, g1): as many as bring at most 32 A entries together
+            const int first = __shfl_sync(FULL, a0, g0);
+            const unsigned fit = __ballot_sync(FULL, lane >= g0 && lane < nr && a1 - first <= 32 && a0 >= first);
+            int g1 = g0 + __ffs(~(fit >> g0)) - 1;
+            if (g1 == g0) {     // one row of more than 32 A entries
+                ++bad;
+                ++g0;
+                continue;
+            }
+            const int last = __shfl_sync(FULL, a1, g1 - 1);
+            int k;
+            const Batch b = load_batch(o, first, last - first, lane, flags, k);
+            const int incl = warp_incl_scan(b.len, lane);
+            const int off = incl - b.len;
+            const unsigned full = __ballot_sync(FULL, b.len > 0);
+            __syncwarp();
+            if (b.len > 0) {
+                OneShare &x = w.share[__popc(full & lanemask_lt())];
+                x.delta = (int)b.bs - off;
+                x.a = o.valA[first + lane];
+            }
+            __syncwarp();
+            int col[ONE_ROWS], cnt[ONE_ROWS];
+#pragma unroll
+            for (int u = 0; u < ONE_ROWS; ++u) {
+                col[u] = -1;
+                cnt[u] = 0;
+                const int i = g0 + u;
+                if (i < g1) {
+                    const int e0 = __shfl_sync(FULL, a0, i) - first, e1 = __shfl_sync(FULL, a1, i) - first;
+                    const int p0 = e0 > 0 ? __shfl_sync(FULL, incl, (e0 - 1) & 31) : 0;
+                    const int p1 = e1 > 0 ? __shfl_sync(FULL, incl, (e1 - 1) & 31) : 0;
+                    const int T = p1 - p0, d = off - p0;
+                    cnt[u] = T;
+                    if (T > 32) ++bad;
+                    else {
+                        // a share that starts at this row's product d sets bit d
+                        const unsigned st = __reduce_or_sync(FULL, (b.len > 0 && d >= 0 && d < T) ? 1u << d : 0u);
+                        if (lane < T) {
+                            const int q = __popc(full & ((1u << (e0 & 31)) - 1u)) + __popc(st & (lanemask_lt() | (1u << lane))) - 1;
+                            const OneShare x = w.share[q];
+                            const int e = x.delta + p0 + lane;
+                            const int c = o.colB[e];
+                            if ((unsigned)c < (unsigned)nb) col[u] = c;
+                            w.ab[u * 32 + lane] = make_double2(x.a, o.valB[e]);
+                        }
+                        products += (unsigned)T;
+                    }
+                }
+            }
+            // the sorts, and the entries of C in order
+            const int base = nout;
+#pragma unroll
+            for (int u = 0; u < ONE_ROWS; ++u) {
+                const int i = g0 + u;
+                if (i < g1 && cnt[u] <= 32) {
+                    K key = col[u] >= 0 ? (((K)(unsigned)col[u] << 5) | (K)(unsigned)lane) : ~(K)0;
+                    key = warp_sort_up(key, lane);
+                    const bool live = key != ~(K)0;
+                    const int c = (int)(key >> 5);
+                    const int pc = __shfl_up_sync(FULL, c, 1);
+                    const bool head = live && (lane == 0 || pc != c);
+                    const unsigned heads = __ballot_sync(FULL, head), lives = __ballot_sync(FULL, live);
+                    const int n = __popc(heads);
+                    if (n != __shfl_sync(FULL, nc, i)) {
+                        ++bad;
+                    } else {
+                        w.src[u * 32 + lane] = (unsigned char)(key & 31u);
+                        if (head) {
+                            const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+                            const int len = later ? __ffs(later) : __popc(lives) - lane;
+                            w.out[nout - base + __popc(heads & lanemask_lt())] =
+                                make_uint2((unsigned)c, (unsigned)(u * 32 + lane) | (unsigned)len << 8);
+                        }
+                        nout += n;
+                    }
+                }
+            }
+            __syncwarp();
+            for (int t = lane; t < nout - base; t += 32) {
+                const uint2 x = w.out[t];
+                const int at = (int)(x.y & 0xffu), row = at & ~31;
+                double acc = 0.0;
+                for (int q = at; q < at + (int)(x.y >> 8); ++q) {
+                    const double2 p = w.ab[row + w.src[q]];
+                    acc = fma(p.x, p.y, acc);
+                }
+                colC[Rb + base + t] = (int)x.x;
+                valC[Rb + base + t] = acc;
+            }
+            g0 = g1;
+        }
+        if (bad && lane == 0) atomicAdd(kept, (unsigned long long)bad);
+    }
+    if (lane == 0) s_prod[warp] = products;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long sum = 0;
+        for (int q = 0; q < ONE_WARPS; ++q) sum += s_prod[q];
+        if (sum) atomicAdd(kept + 1, sum);
+        // the last CTA reports to the host and clears the counts for the next call
+        __threadfence();
+        if (atomicAdd(&rep->done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            volatile SmallReport *v = rep;
+            host[0] = (long long)v->kept[0];
+            host[1] = (long long)v->kept[1];
+            for (int f = 0; f < FLAG_COUNT; ++f) {
+                host[2 + f] = v->flags[f];
+                v->flags[f] = 0;
+            }
+            v->kept[0] = v->kept[1] = 0;
+            v->done = 0;
+            __threadfence_system();
+        }
     }
 }
 
@@ -421,7 +612,7 @@ cudaError_t small_count(Pool &pool, const SmallOperands &o, int *rowcnt, unsigne
 }
 
 cudaError_t small_fill(Pool &pool, const SmallOperands &o, const long long *rowptrC, long long cap, int *colC,
-                       double *valC, int *flags, unsigned long long *kept, void *rp_out, int rp_bits, bool one_round)
+                       double *valC, int *flags, unsigned long long *kept, void *rp_out, int rp_bits)
 {
     const int m = o.m;
     if (m <= 0) {   // C's row pointer is the single 0
@@ -429,12 +620,25 @@ cudaError_t small_fill(Pool &pool, const SmallOperands &o, const long long *rowp
         return cudaMemsetAsync(rp_out, 0, rp_bits == 64 ? 8 : 4, pool.stream);
     }
     const unsigned grid = (unsigned)((m + SH_WARPS - 1) / SH_WARPS);
-    if (one_round && kept)
-        k_small_fill<true><<<grid, SH_WARPS * 32, 0, pool.stream>>>(o, rowptrC, cap, colC, valC, flags, kept, rp_out,
-                                                                    rp_bits);
-    else
-        k_small_fill<false><<<grid, SH_WARPS * 32, 0, pool.stream>>>(o, rowptrC, cap, colC, valC, flags, kept, rp_out,
-                                                                     rp_bits);
+    k_small_fill<<<grid, SH_WARPS * 32, 0, pool.stream>>>(o, rowptrC, cap, colC, valC, flags, kept, rp_out, rp_bits);
+    ::tsg::count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t small_fill_one(Pool &pool, const SmallOperands &o, const long long *rowptrC, long long cap, int *colC,
+                           double *valC, SmallReport *rep, long long *host, void *rp_out, int rp_bits)
+{
+    // one row a warp while the rows do not fill the SMs' warps (1,024 rows:
+    // 8.7 us, 11.3 with four); 32-bit keys when B's columns leave room for
+    // the 5 bits of f
+    const int rows = o.m < 20000 ? 1 : 4;
+    const unsigned grid = (unsigned)((o.m + ONE_WARPS * rows - 1) / (ONE_WARPS * rows));
+    auto run = [&](auto kernel) {
+        kernel<<<grid, ONE_WARPS * 32, 0, pool.stream>>>(o, rowptrC, cap, colC, valC, rep, host, rp_out, rp_bits);
+    };
+    const bool narrow = o.nb <= (1 << 26);
+    if (rows == 1) narrow ? run(k_small_fill_one<1, unsigned>) : run(k_small_fill_one<1, unsigned long long>);
+    else narrow ? run(k_small_fill_one<4, unsigned>) : run(k_small_fill_one<4, unsigned long long>);
     ::tsg::count_launch();
     return cudaGetLastError();
 }
