@@ -1025,7 +1025,19 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     // SMs are full (512 mixed products: 30.7 ms with 64, 36.6 with 32, 39.1 with 200)
     g.each = h.products > 24000000 ? 64.0f : 32.0f;
     if (!items) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's items)");
-    CUDA_OK(row_symbolic(pool, g, prod, heavy, h.heavy, h.width, rowcnt, items, (unsigned)cap, rs->nitems, ctx->side,
+    {   // the rows' bitmaps kept for the numeric pass: at most a sixteenth of the free device memory
+        const long long bytes = 128ll * (long long)h.blocks;
+        size_t free_b = 0, total_b = 0;
+        if (h.blocks < (1ull << 31) &&
+            (bytes <= (64ll << 20) ||
+             (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= (long long)(free_b / 16)))) {
+            g.bits = sc.get<unsigned>(32ll * (long long)h.blocks);
+            g.bitoff = sc.get<int>(P.m);
+            if (!g.bits || !g.bitoff) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's bitmaps)");
+        }
+        cudaGetLastError();
+    }
+    CUDA_OK(row_symbolic(pool, g, prod, heavy, h.heavy, h.width, rowcnt, items, (unsigned)cap, rs, ctx->side,
                          ctx->fork, ctx->join));
     CUDA_OK(scan_i32_to_i64(pool, rowcnt, P.rowptrC, P.m, ctx->dflags));
     CUDA_OK(cudaMemcpyAsync(ctx->dstat + ST_NNZC, P.rowptrC + P.m, sizeof(long long), cudaMemcpyDeviceToDevice,

@@ -14,10 +14,11 @@
 //   k_row_symbolic  per row of C a bitmap of its columns in shared memory, its
 //                   entries per block, and from them its items: one for a
 //                   light row, else runs of blocks that close at ITEM_T
-//                   entries or ITEM_BLKS blocks
+//                   entries or ITEM_BLKS blocks; dense enough bitmaps are kept
 //   (the look-back scan of the row counts gives C's row pointer)
-//   k_row_numeric   per item: the bitmap of its columns and running counts (a
-//                   column's position = count + popc), then its products in
+//   k_row_numeric   per item: the bitmap of its columns (kept, or marked again)
+//                   and running counts (a column's position = count + popc),
+//                   then its products in
 //                   steps, one A entry's B entries each: one fma a product on
 //                   its position's accumulator in shared memory
 // The steps follow one another in A's row order and a step's columns differ,
@@ -27,14 +28,16 @@
 // k_count_descents; the tiled path takes the others).
 //
 // Measured on GB300, before (tiled) and after, whole call on the device:
-//   R-MAT 2^12 x 8 A*A^T 1,190 -> 431 us, 2^15 x 16 A*A^T 8.4 -> 2.3 ms,
-//   2^16 x 12 A*A 12.9 -> 3.4 ms, 2^18 x 16 A*A^T 80 -> 42 ms;
-//   uniform 120,007 x 80,021 x 100,003, 16 and 12 a row: 10.3 -> 2.0 ms.
-// What bounds it (2^15, counters): k_row_numeric, 2/3 of the time, is bound
-// by issue and by the latency of a step's chain (B's entry, its word, its
-// accumulator, the fma): some 60 instructions a step at 1.1 to 1.6 a clock
-// and SM, FP64 pipe 20-30 % busy.  k_row_symbolic is bound by its bitmap's
-// shared-memory accesses.
+//   R-MAT 2^12 x 8 A*A^T 1,190 -> 414 us, 2^15 x 16 A*A^T 8.4 -> 2.2 ms,
+//   2^16 x 12 A*A 12.9 -> 3.0 ms, 2^18 x 16 A*A^T 80 -> 35.6 ms;
+//   uniform 120,007 x 80,021 x 100,003, 16 and 12 a row: 10.3 -> 2.0 ms;
+//   512 mixed products of 64 to 16,384 rows: 41.7 -> 24.5 ms.
+// What bounds it (2^15, counters): k_row_numeric, 2/3 of the time, by issue
+// and by the latency of a step's chain (B's entry, its word, its accumulator,
+// the fma): 28 instructions a step and 7 to stage it, 1.1 to 1.6 a clock and
+// SM, FP64 pipe 20-30 % busy; marking an item's columns again cost another 28
+// a step (2^18: 41.0 ms without kept bitmaps).  k_row_symbolic is bound by its
+// bitmap's shared-memory accesses.
 // Tried without gain: products flattened 32 at a time over an item's shares,
 // lanes that meet ordered by rank (2^18: 77 ms; R-MAT's columns meet in
 // nearly every round); items of 6,144 entries as a CTA's, 128 entries a step
@@ -83,10 +86,10 @@ __global__ void k_row_extents(const long long *__restrict__ rpB, const int *__re
 __global__ void __launch_bounds__(256)
 k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, int *heavy, RowStat *stat)
 {
-    __shared__ unsigned long long s_p[8], s_i[8];
+    __shared__ unsigned long long s_p[8], s_i[8], s_b[8];
     __shared__ int s_w[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned long long sp = 0, si = 0;
+    unsigned long long sp = 0, si = 0, sb = 0;
     int width = 0;
     for (long long r = blockIdx.x * 8ll + warp; r < g.m; r += gridDim.x * 8ll) {
         long long p = 0;
@@ -118,6 +121,7 @@ k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, in
             const int nb = hi < lo ? 0 : hi - lo + 1;
             rng[r] = make_int2(nb ? lo : 0, nb ? hi + 1 : 0);
             width = max(width, nb);
+            if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
             sp += (unsigned long long)p;
             si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
             if ((p > LIGHT_ROW || nb > SYM_BLKS) && !stat->cuts) stat->cuts = 1;
@@ -127,14 +131,15 @@ k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, in
             }
         }
     }
-    if (lane == 0) { s_p[warp] = sp; s_i[warp] = si; s_w[warp] = width; }
+    if (lane == 0) { s_p[warp] = sp; s_i[warp] = si; s_b[warp] = sb; s_w[warp] = width; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned long long a = 0, b = 0;
+        unsigned long long a = 0, b = 0, c = 0;
         int w = 0;
-        for (int q = 0; q < 8; ++q) { a += s_p[q]; b += s_i[q]; w = max(w, s_w[q]); }
+        for (int q = 0; q < 8; ++q) { a += s_p[q]; b += s_i[q]; c += s_b[q]; w = max(w, s_w[q]); }
         atomicAdd(&stat->products, a);
         atomicAdd(&stat->items, b);
+        atomicAdd(&stat->blocks, c);
         if (w > *(volatile int *)&stat->width) atomicMax(&stat->width, w);
     }
 }
@@ -181,8 +186,10 @@ struct HeavyRows {
 template <int NT>
 __global__ void __launch_bounds__(NT)
 k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRows heavy, int width, int *rowcnt,
-               int4 *items, unsigned cap, unsigned *nitems)
+               int4 *items, unsigned cap, RowStat *stat)
 {
+    unsigned *nitems = stat->nitems;
+    __shared__ unsigned s_bit;
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned s_sym[];
     const int r = heavy.list ? heavy.row(blockIdx.x) : blockIdx.x;
@@ -198,6 +205,11 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
     unsigned *bits = s_sym;
     int *cnt = reinterpret_cast<int *>(s_sym + min(width, SYM_BLKS) * (ROW_BLK / 32));
     const long long a0 = g.rpA[r], a1 = g.rpA[r + 1];
+    const bool keep = g.bits && p >= KEEP_BITS * (long long)nblk;
+    if (g.bits && tid == 0) {      // the row's place among the kept bitmaps
+        if (keep) s_bit = atomicAdd(&stat->bitblk, (unsigned)nblk);
+        g.bitoff[r] = keep ? (int)s_bit : -1;
+    }
     for (int wb = 0; wb < nblk; wb += SYM_BLKS) {
         const int nb = min(SYM_BLKS, nblk - wb);
         const int c0 = (first + wb) << ROW_BLK_LOG;
@@ -276,6 +288,10 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
             }
         }
         __syncthreads();
+        if (keep) {
+            uint4 *out = reinterpret_cast<uint4 *>(g.bits + ((long long)s_bit + wb) * (ROW_BLK / 32));
+            for (int t = tid; t < nb * (ROW_BLK / 128); t += NT) out[t] = reinterpret_cast<const uint4 *>(bits)[t];
+        }
         for (int j = warp; j < nb; j += NW) {
             const unsigned c = __reduce_add_sync(FULL, (unsigned)__popc(bits[j * (ROW_BLK / 32) + lane]));
             if (lane == 0) cnt[wb + j] = (int)c;
@@ -386,8 +402,11 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
     const long long a0 = g.rpA[r], a1 = g.rpA[r + 1];
     const int2 rng = g.rng[r];
     const bool whole = nb == rng.y - rng.x;      // the row's only item: whole B rows
-    for (int w = tid; w < (dense ? nb * (ROW_BLK / 16) : nw / 2); w += NT)
-        reinterpret_cast<uint4 *>(tag)[w] = make_uint4(0u, 0u, 0u, 0u);
+    // the symbolic pass's bitmap, when it is no longer than the item's values
+    const int bit = !dense && g.bits && KEEP_BITS * nb <= z ? g.bitoff[r] : -1;
+    if (bit < 0)
+        for (int w = tid; w < (dense ? nb * (ROW_BLK / 16) : nw / 2); w += NT)
+            reinterpret_cast<uint4 *>(tag)[w] = make_uint4(0u, 0u, 0u, 0u);
     for (int t = tid; t < (dense ? nb * ROW_BLK : z); t += NT) acc[t] = 0.0;
     int nk = -1, ns = 0, ne = 0;       // the next NT A entries' B rows and shares, loaded ahead
     double nav = 0.0;
@@ -445,9 +464,10 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
         sync();
     };
     if (!dense) {
-        // the columns: a warp takes every NW-th group of steps, or, with
-        // steps wider than a warp, every NW-th step
-        walk([&](int n) {
+        // the columns: kept by the symbolic pass, or marked again: a warp takes
+        // every NW-th group of steps, or, with steps wider than a warp, every
+        // NW-th step
+        if (bit < 0) walk([&](int n) {
             auto mark = [&](int c) { atomicOr(&word[(c - c0) >> 5].x, 1u << (c & 31)); };
             if constexpr (NT == 32) {
                 for (int i = 0; i < n; i += ROW_GROUP) {
@@ -482,14 +502,26 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
         // round; then the warps' totals
         const int per = ((nw + NW - 1) / NW + 63) & ~63, w1 = min(nw, (warp + 1) * per);
         int run = 0;
-        for (int w = warp * per + 2 * lane; w - 2 * lane < w1; w += 64) {
-            uint4 x = w < w1 ? *reinterpret_cast<const uint4 *>(word + w) : make_uint4(0u, 0u, 0u, 0u);
+        auto rank = [&](int w, uint4 x) {
             const int n0 = __popc(x.x), sum = n0 + __popc(x.z);
             const int incl = warp_incl_scan(sum, lane);
             x.y = (unsigned)(run + incl - sum);
             x.w = x.y + (unsigned)n0;
             run += __shfl_sync(FULL, incl, 31);
             if (w < w1) *reinterpret_cast<uint4 *>(word + w) = x;
+        };
+        if (bit < 0) {
+            for (int w = warp * per + 2 * lane; w - 2 * lane < w1; w += 64)
+                rank(w, w < w1 ? *reinterpret_cast<const uint4 *>(word + w) : make_uint4(0u, 0u, 0u, 0u));
+        } else {
+            const uint2 *kept = reinterpret_cast<const uint2 *>(g.bits + ((long long)bit + j0 - rng.x) * (ROW_BLK / 32));
+            for (int w = warp * per + 2 * lane; w - 2 * lane < w1; w += 4 * 64) {
+                uint2 x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) x[u] = w + 64 * u < w1 ? kept[(w >> 1) + 32 * u] : make_uint2(0u, 0u);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) rank(w + 64 * u, make_uint4(x[u].x, 0u, x[u].y, 0u));
+            }
         }
         int total = run;
         if constexpr (NT > 32) {
@@ -692,7 +724,7 @@ cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut)
 }
 
 cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const unsigned *nheavy,
-                         int width, int *rowcnt, int4 *items, unsigned cap, unsigned *nitems, cudaStream_t side,
+                         int width, int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
                          cudaEvent_t fork, cudaEvent_t join)
 {
     cudaStream_t s = pool.stream;
@@ -707,11 +739,11 @@ cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const in
         HeavyRows hl = h;
         hl.list = heavy;
         hl.m = g.m;
-        k_row_symbolic<1024><<<(unsigned)total, 1024, sm, side>>>(g, prod, ROW_HEAVY, INT_MAX, hl, width, rowcnt, items, cap, nitems);
+        k_row_symbolic<1024><<<(unsigned)total, 1024, sm, side>>>(g, prod, ROW_HEAVY, INT_MAX, hl, width, rowcnt, items, cap, stat);
         ::tsg::count_launch();
     }
-    k_row_symbolic<256><<<(unsigned)g.m, 256, sm, s>>>(g, prod, ROW_TINY, ROW_HEAVY, h, width, rowcnt, items, cap, nitems);
-    k_row_symbolic<64><<<(unsigned)g.m, 64, sm, side>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, nitems);
+    k_row_symbolic<256><<<(unsigned)g.m, 256, sm, s>>>(g, prod, ROW_TINY, ROW_HEAVY, h, width, rowcnt, items, cap, stat);
+    k_row_symbolic<64><<<(unsigned)g.m, 64, sm, side>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, stat);
     ::tsg::count_launch();
     ::tsg::count_launch();
     e = cudaGetLastError();

@@ -9,6 +9,10 @@ constexpr int ITEM_T = 1024;                  // an item closes once its row's e
 constexpr int ITEM_CAP = ITEM_T + ROW_BLK;    // entries of an item at most (a block adds at most ROW_BLK)
 constexpr int ITEM_BLKS = 16;                 // blocks of an item at most
 constexpr int LIGHT_ROW = 4096, LIGHT_BLKS = 256;   // rows of so few entries: one item per so many blocks
+constexpr int KEEP_BITS = 16;               // products a block from which a row's bitmap is kept for the numeric
+                                              // pass (and entries a block from which an item reads it: 128 bytes a
+                                              // block against 8 an entry; with none of its own, uniform rows of 192
+                                              // products over 98 blocks: 2.0 ms marked again, 2.7 read back)
 constexpr int SYM_BLKS = 256;                 // blocks of the symbolic bitmap at a time (32 KB)
 constexpr int ROW_MAX_BLKS = 4096;            // blocks of a row's columns at most (4 M columns)
 constexpr int ROW_HEAVY = 1 << 15;            // rows of more products take a CTA of 1,024 threads
@@ -68,6 +72,10 @@ struct RowArgs {
     const int *base = nullptr;
     int width = 0;
     const int *coloff = nullptr;              // batches: per 16 rows of C, subtracted from its columns
+    // The rows' column bitmaps, kept by k_row_symbolic for k_row_numeric when
+    // there is room: row r's 32 words a block from block bitoff[r] on (-1: not kept).
+    unsigned *bits = nullptr;
+    int *bitoff = nullptr;
     __device__ __forceinline__ const int *cuts(int k, int j) const {   // B row k's, from block j on
         return cut + (long long)k * (width + 1) + (j - (base ? base[k >> 4] : 0));
     }
@@ -80,7 +88,8 @@ struct RowStat {
     int width;                                // blocks of the widest row
     int cuts;                                 // a row needs the cut table (more than one item or window)
     int bad;                                  // a column of A outside B's rows
-    int pad;
+    unsigned bitblk;                          // row_symbolic: blocks of kept bitmaps handed out
+    unsigned long long blocks;                // blocks of all rows
     unsigned nitems[ITEM_CLASSES];            // row_symbolic: items of each class
 };
 
@@ -91,7 +100,7 @@ cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int
 cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut);
 // items: ITEM_CLASSES lists of cap
 cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const unsigned *nheavy,
-                         int width, int *rowcnt, int4 *items, unsigned cap, unsigned *nitems, cudaStream_t side,
+                         int width, int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
                          cudaEvent_t fork, cudaEvent_t join);
 cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigned cap, const unsigned *n,
                         const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
