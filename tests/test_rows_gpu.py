@@ -31,6 +31,12 @@ def _rows(m, n, lens, seed):
     return CSR(m, n, rp, col.astype(np.int32), rng.uniform(-1.0, 1.0, int(rp[-1])))
 
 
+def _spread(X, f):
+    """X's columns f apart."""
+    from tilespgemm_gb300.api import CSR
+    return CSR(X.m, X.n * f, X.rowptr, X.col * np.int32(f), X.val)
+
+
 def _cases():
     from tilespgemm_gb300 import matrices as M
     return {
@@ -45,6 +51,10 @@ def _cases():
         "heavy_windows": (_rows(5, 400, [380, 40], 16), _rows(400, 290003, [3000, 0, 9000], 17), "AB"),
         "dense_blocks": (_rows(40, 200, [150, 60], 18), _rows(200, 5000, [2500, 4000, 8], 19), "AB"),
         "full_rows": (_rows(6, 90, [90], 20), _rows(90, 2049, [2049], 21), "AB"),
+        "sort_classes": (_rows(700, 60, [1], 22),
+                         _rows(60, 120007, [1, 31, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 0], 23), "AB"),
+        "sort_batches": (_rows(150, 300, [64, 33, 32, 65, 130, 7], 24), _rows(300, 100003, [0, 4, 8, 3, 1], 25), "AB"),
+        "sort_repeats": (_rows(200, 50, [4, 3, 1, 5], 26), _spread(_rows(50, 150, [128, 40, 100], 27), 900), "AB"),
         "rmat9": (M.rmat(9, 8, seed=3), None, "AAT"),
         "rmat12": (M.rmat(12, 8, seed=4), None, "AA"),
         "stencil": (M.stencil_27(11, seed=2), None, "AAT"),

@@ -990,6 +990,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     g.m = P.m; g.k = P.k; g.n = P.n; g.nblk = ceil_div_i(P.n, ROW_BLK);
     g.rpA = P.rpA; g.rpB = P.rpB; g.colA = P.colA; g.colB = P.colB; g.valA = P.valA; g.valB = P.valB;
     g.width = g.nblk;
+    g.sort_max = P.n <= SORT_COLS ? SORT_MAX : 0;
     if (batch) { g.base = batch->base; g.width = batch->width; g.coloff = batch->coloff; }
     Scratch sc(pool);
     static_assert(sizeof(RowStat) <= 8 * BS_SLOTS, "the row path's statistics fit the bins' slots");
@@ -1004,8 +1005,8 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     if (r) return r;
     memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
     const long long cap = std::max<long long>((long long)h.items, 1);
-    if (h.bad || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS) return TSG_OK;
-    if (h.cuts) {   // the cut table: at most a sixteenth of the free device memory
+    if ((h.seen & SEEN_BAD) || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS) return TSG_OK;
+    if (h.seen & SEEN_CUTS) {   // the cut table: at most a sixteenth of the free device memory
         const long long n = (long long)P.k * (g.width + 1);
         size_t free_b = 0, total_b = 0;
         if (4 * n > (64ll << 20) &&
@@ -1037,7 +1038,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
         }
         cudaGetLastError();
     }
-    CUDA_OK(row_symbolic(pool, g, prod, heavy, h.heavy, h.width, rowcnt, items, (unsigned)cap, rs, ctx->side,
+    CUDA_OK(row_symbolic(pool, g, prod, heavy, h, rowcnt, items, (unsigned)cap, rs, ctx->side,
                          ctx->fork, ctx->join));
     CUDA_OK(scan_i32_to_i64(pool, rowcnt, P.rowptrC, P.m, ctx->dflags));
     CUDA_OK(cudaMemcpyAsync(ctx->dstat + ST_NNZC, P.rowptrC + P.m, sizeof(long long), cudaMemcpyDeviceToDevice,
@@ -1054,7 +1055,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     val = pool.out_n<double>(P.nnzC);
     if (!col || !val) return fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
     P.wait_values(ctx->stream);
-    CUDA_OK(row_numeric(pool, g, items, (unsigned)cap, h.nitems, P.rowptrC, col, val, ctx->dflags, ctx->side,
+    CUDA_OK(row_numeric(pool, g, prod, items, (unsigned)cap, h, P.rowptrC, col, val, ctx->dflags, ctx->side,
                         ctx->fork, ctx->join));
     taken = true;
     return TSG_OK;

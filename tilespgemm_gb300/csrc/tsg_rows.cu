@@ -57,6 +57,16 @@ namespace tsg {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
+// Rows sorted in place of a bitmap: the bitmap costs by the row's blocks, the
+// sort by its products.  The line lies between spans that were measured, call
+// with bitmaps / sorted: 64 blocks (R-MAT 2^16 x 12 A*A) 3,008 / 3,155 us, 32
+// (R-MAT 2^15 x 16 A*A^T) 2,229 / 2,311, 98 (uniform, 192 products a row)
+// 2,083 / 727, 256 (R-MAT 2^18 x 16) 35,674 / 35,066.
+__device__ __forceinline__ bool sorted_row(const RowArgs &g, long long p, int nb)
+{
+    return p > 0 && p <= g.sort_max && nb >= SORT_NB;
+}
+
 // The products of every step-th row of C, times step (one warp a row).
 __global__ void __launch_bounds__(256)
 k_row_sample(RowArgs g, int step, unsigned long long *out)
@@ -115,16 +125,23 @@ k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, in
         p = warp_sum_ll(p);
         lo = __reduce_min_sync(FULL, lo);
         hi = __reduce_max_sync(FULL, hi);
-        if (out) stat->bad = 1;
+        out = __any_sync(FULL, out);
         if (lane == 0) {
+            unsigned seen = 0;
+            sp += (unsigned long long)p;
             prod[r] = (int)min(p, (long long)INT_MAX);
             const int nb = hi < lo ? 0 : hi - lo + 1;
             rng[r] = make_int2(nb ? lo : 0, nb ? hi + 1 : 0);
-            width = max(width, nb);
-            if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
-            sp += (unsigned long long)p;
-            si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
-            if ((p > LIGHT_ROW || nb > SYM_BLKS) && !stat->cuts) stat->cuts = 1;
+            if (sorted_row(g, p, nb)) {          // no bitmap, no item
+                seen = p > 256 ? SEEN_SORT << 2 : p > 128 ? SEEN_SORT << 1 : SEEN_SORT;
+            } else {
+                width = max(width, nb);
+                if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
+                si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
+                if (p > LIGHT_ROW || nb > SYM_BLKS) seen = SEEN_CUTS;
+            }
+            if (out) seen |= SEEN_BAD;
+            if (seen & ~*(volatile unsigned *)&stat->seen) atomicOr(&stat->seen, seen);
             if (p > ROW_HEAVY) {
                 const int c = heavy_class(p);
                 heavy[(long long)c * g.m + atomicAdd(stat->heavy + c, 1u)] = (int)r;
@@ -196,12 +213,13 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int p = prod[r];
     if (p <= p0 || p > p1) {
-        if (p == 0 && p0 == 0 && tid == 0) rowcnt[r] = 0;
+        if (p == 0 && p1 == ROW_TINY && tid == 0) rowcnt[r] = 0;
         return;
     }
     // the row's blocks: first, then counted from it
     const int2 rng = g.rng[r];
     const int first = rng.x, nblk = rng.y - rng.x;
+    if (sorted_row(g, p, nblk)) return;
     unsigned *bits = s_sym;
     int *cnt = reinterpret_cast<int *>(s_sym + min(width, SYM_BLKS) * (ROW_BLK / 32));
     const long long a0 = g.rpA[r], a1 = g.rpA[r + 1];
@@ -667,6 +685,197 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
     for (int t = tid; t < z; t += NT) colC[Rb + t] = ccol[t];
 }
 
+// ---- rows of few products: sorted in registers ---------------------------------
+//
+// A row of up to SORT_MAX products needs no bitmap of its span: one warp
+// sorts the keys (column, product) -- E a lane, a bitonic network, strides
+// below E inside a lane -- and a column's products then lie side by side in
+// product order: counted for C's row, or applied to its entry in that order.
+// The product number in the low bits leaves 23 bits for the column.
+// Bound by issue (the network: 650 instructions for 256 keys); the bitmap of
+// such a row took 3,000 over 98 blocks, and 27 KB of shared memory.
+// Measured on GB300: uniform 120,007 x 80,021 x 100,003, 192 products a row over
+// 98 blocks: 2,080 -> 727 us a call (k_row_sort 140 us to count, 227 to fill).
+constexpr int SORT_WARPS = 4;
+
+struct __align__(16) Share {     // one A entry's B row: entry f + delta for the row's product f
+    int delta, pad;
+    double a;
+};
+
+template <int E, bool FILL>
+struct SortSmem {
+    unsigned key[32 * E];
+    Share share[32];
+};
+template <int E>
+struct SortSmem<E, true> {
+    unsigned key[32 * E];
+    Share share[32];
+    double2 ab[32 * E];             // product: A's and B's value
+    unsigned short at[32 * E + 2];  // C entry: its first sorted product
+};
+
+template <int E>
+__device__ __forceinline__ void sort_keys(unsigned (&x)[E], int lane)
+{
+#pragma unroll
+    for (int k = 2; k < E; k <<= 1)          // inside a lane, both directions
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if ((e & j) == 0) {
+                    const unsigned lo = min(x[e], x[e | j]), hi = max(x[e], x[e | j]);
+                    x[e] = (e & k) ? hi : lo;
+                    x[e | j] = (e & k) ? lo : hi;
+                }
+    unsigned flip = 0;
+#pragma unroll
+    for (int k = E; k <= 32 * E; k <<= 1) {
+        // lanes that sort downwards hold their keys complemented
+        const unsigned down = k < 32 * E && (lane & (k / E)) ? 0xffffffffu : 0u;
+        const unsigned turn = flip ^ down;
+        flip = down;
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[e] ^= turn;
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= E) {
+                const bool up = lane & (j / E);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const unsigned y = __shfl_xor_sync(FULL, x[e], j / E);
+                    x[e] = up ? max(x[e], y) : min(x[e], y);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e)
+                    if ((e & j) == 0) {
+                        const unsigned lo = min(x[e], x[e | j]), hi = max(x[e], x[e | j]);
+                        x[e] = lo;
+                        x[e | j] = hi;
+                    }
+            }
+        }
+    }
+}
+
+// One warp per row of C with products in (lo, 32 E].
+template <int E, bool FILL>
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+k_row_sort(RowArgs g, const int *__restrict__ prod, int lo, int *rowcnt, const long long *__restrict__ rowptrC,
+           int *__restrict__ colC, double *__restrict__ valC, int *flags)
+{
+    __shared__ SortSmem<E, FILL> s_w[SORT_WARPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = blockIdx.x * SORT_WARPS + warp;
+    if (r >= g.m) return;
+    const int p = prod[r];
+    if (p <= lo || p > 32 * E) return;
+    const int2 rng = g.rng[r];
+    if (!sorted_row(g, p, rng.y - rng.x)) return;
+    SortSmem<E, FILL> &w = s_w[warp];
+    for (int t = p + lane; t < 32 * E; t += 32) w.key[t] = 0xffffffffu;
+    const long long a1 = g.rpA[r + 1];
+    int f0 = 0;                                     // products before this batch of A entries
+    for (long long a = g.rpA[r]; a < a1; a += 32) {
+        int s = 0, len = 0;
+        double av = 0.0;
+        if (a + lane < a1) {
+            const int k = g.colA[a + lane];
+            if (FILL) av = g.valA[a + lane];
+            s = (int)g.rpB[k];
+            len = (int)g.rpB[k + 1] - s;
+        }
+        const int incl = warp_incl_scan(len, lane), off = incl - len, T = __shfl_sync(FULL, incl, 31);
+        const unsigned live = __ballot_sync(FULL, len > 0);
+        __syncwarp();
+        if (len > 0) {
+            Share &x = w.share[__popc(live & lanemask_lt())];
+            x.delta = s - off;
+            x.a = av;
+        }
+        __syncwarp();
+        int done = 0;
+        for (int base = 0; base < T; base += 32) {
+            // a share that starts in this round sets the bit of the lane it starts at
+            const int d = off - base;
+            const unsigned m = __reduce_or_sync(FULL, (len > 0 && (unsigned)d < 32u) ? 1u << d : 0u);
+            const int q = done + __popc(m & (lanemask_lt() | (1u << lane))) - 1;
+            done += __popc(m);
+            const int f = base + lane;
+            if (f < T) {
+                const int e = w.share[q].delta + f;
+                w.key[f0 + f] = (unsigned)g.colB[e] << SORT_BITS | (unsigned)(f0 + f);
+                if constexpr (FILL) w.ab[f0 + f] = make_double2(w.share[q].a, g.valB[e]);
+            }
+        }
+        f0 += T;
+    }
+    __syncwarp();
+    unsigned x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = w.key[lane * E + e];
+    sort_keys<E>(x, lane);
+    // the first product of each column starts an entry of C
+    unsigned before = __shfl_up_sync(FULL, x[E - 1], 1);
+    unsigned heads = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const bool first = lane == 0 && e == 0;
+        if (x[e] != 0xffffffffu && (first || (x[e] >> SORT_BITS) != (before >> SORT_BITS))) heads |= 1u << e;
+        before = x[e];
+    }
+    const int n = __popc(heads);
+    if constexpr (!FILL) {
+        const int z = (int)__reduce_add_sync(FULL, (unsigned)n);
+        if (lane == 0) rowcnt[r] = z;
+    } else {
+        const int incl = warp_incl_scan(n, lane), z = __shfl_sync(FULL, incl, 31);
+        int o = incl - n;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            w.key[lane * E + e] = x[e];
+            if ((heads >> e) & 1u) w.at[o++] = (unsigned short)(lane * E + e);
+        }
+        if (lane == 0) w.at[z] = (unsigned short)p;
+        __syncwarp();
+        const long long Rb = rowptrC[r];
+        if (rowptrC[r + 1] - Rb != z) {
+            if (lane == 0) set_flag(flags, FLAG_INTERNAL);
+            return;
+        }
+        const int shift = g.coloff ? g.coloff[r >> 4] : 0;
+        for (int t = lane; t < z; t += 32) {
+            const int q0 = w.at[t], q1 = w.at[t + 1];
+            unsigned k = w.key[q0];
+            colC[Rb + t] = (int)(k >> SORT_BITS) - shift;
+            double acc = 0.0;
+            for (int q = q0; q < q1; ++q) {
+                const double2 v = w.ab[w.key[q] & (unsigned)(SORT_MAX - 1)];
+                acc = fma(v.x, v.y, acc);
+            }
+            valC[Rb + t] = acc;
+        }
+    }
+}
+
+template <bool FILL>
+cudaError_t sort_rows(cudaStream_t s, const RowArgs &g, const int *prod, const RowStat &h, int *rowcnt,
+                      const long long *rowptrC, int *colC, double *valC, int *flags)
+{
+    const unsigned grid = (unsigned)((g.m + SORT_WARPS - 1) / SORT_WARPS);
+    auto run = [&](auto kernel, int lo) {
+        kernel<<<grid, SORT_WARPS * 32, 0, s>>>(g, prod, lo, rowcnt, rowptrC, colC, valC, flags);
+        ::tsg::count_launch();
+    };
+    if (h.seen & SEEN_SORT << 2) run(k_row_sort<16, FILL>, 256);
+    if (h.seen & SEEN_SORT << 1) run(k_row_sort<8, FILL>, 128);
+    if (h.seen & SEEN_SORT) run(k_row_sort<4, FILL>, 0);
+    return cudaGetLastError();
+}
+
 size_t sym_smem(int width) { return (size_t)std::min(width, SYM_BLKS) * (ROW_BLK / 8) + 4 * ((size_t)width + 1); }
 
 unsigned warps_grid(long long rows) { return (unsigned)std::min<long long>(std::max<long long>((rows + 7) / 8, 1), 152 * 32); }
@@ -723,15 +932,16 @@ cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut)
     return cudaGetLastError();
 }
 
-cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const unsigned *nheavy,
-                         int width, int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
+cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const RowStat &hs,
+                         int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
                          cudaEvent_t fork, cudaEvent_t join)
 {
     cudaStream_t s = pool.stream;
+    const int width = hs.width;
     const size_t sm = sym_smem(width);
     HeavyRows h;
     int total = 0;
-    for (int c = 0; c < HEAVY_CLASSES; ++c) total += h.n[c] = (int)nheavy[c];
+    for (int c = 0; c < HEAVY_CLASSES; ++c) total += h.n[c] = (int)hs.heavy[c];
     cudaError_t e = cudaEventRecord(fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
     if (e != cudaSuccess) return e;
@@ -742,17 +952,22 @@ cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const in
         k_row_symbolic<1024><<<(unsigned)total, 1024, sm, side>>>(g, prod, ROW_HEAVY, INT_MAX, hl, width, rowcnt, items, cap, stat);
         ::tsg::count_launch();
     }
-    k_row_symbolic<256><<<(unsigned)g.m, 256, sm, s>>>(g, prod, ROW_TINY, ROW_HEAVY, h, width, rowcnt, items, cap, stat);
-    k_row_symbolic<64><<<(unsigned)g.m, 64, sm, side>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, stat);
-    ::tsg::count_launch();
-    ::tsg::count_launch();
-    e = cudaGetLastError();
+    if (width > 0) {
+        k_row_symbolic<256><<<(unsigned)g.m, 256, sm, s>>>(g, prod, ROW_TINY, ROW_HEAVY, h, width, rowcnt, items, cap, stat);
+        k_row_symbolic<64><<<(unsigned)g.m, 64, sm, side>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, stat);
+        ::tsg::count_launch();
+        ::tsg::count_launch();
+    } else {      // every row is sorted, or empty
+        e = cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)g.m, s);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = sort_rows<false>(s, g, prod, hs, rowcnt, nullptr, nullptr, nullptr, nullptr);
     cudaError_t j = cudaEventRecord(join, side);
     if (j == cudaSuccess) j = cudaStreamWaitEvent(s, join, 0);
     return e == cudaSuccess ? j : e;
 }
 
-cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigned cap, const unsigned *n,
+cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int *prod, const int4 *items, unsigned cap, const RowStat &h,
                         const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
                         cudaEvent_t fork, cudaEvent_t join)
 {
@@ -766,9 +981,10 @@ cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigne
         const int c = order[q];
         cudaStream_t on = q % 2 ? s : side;
         const int4 *list = items + (long long)c * cap;
-        e = c < CLASS_WARP ? numeric_class<32>(on, g, list, n[c], c, rowptrC, colC, valC, flags)
-                           : numeric_class<NT_WIDE>(on, g, list, n[c], c, rowptrC, colC, valC, flags);
+        e = c < CLASS_WARP ? numeric_class<32>(on, g, list, h.nitems[c], c, rowptrC, colC, valC, flags)
+                           : numeric_class<NT_WIDE>(on, g, list, h.nitems[c], c, rowptrC, colC, valC, flags);
     }
+    if (e == cudaSuccess) e = sort_rows<true>(s, g, prod, h, nullptr, rowptrC, colC, valC, flags);
     cudaError_t j = cudaEventRecord(join, side);
     if (j == cudaSuccess) j = cudaStreamWaitEvent(s, join, 0);
     return e == cudaSuccess ? j : e;

@@ -58,11 +58,16 @@ static_assert(LIGHT_BLKS * (ROW_BLK / 4) + LIGHT_ROW * 12 <= class_smem(6), "eve
 static_assert(LIGHT_ROW * 2 * 9 <= class_smem(6) && ITEM_CAP * 2 * 9 <= class_smem(6), "dense items fit");
 static_assert(ITEM_BLKS * (ROW_BLK / 4) + ITEM_CAP * 12 <= class_smem(3), "every other item fits a warp's classes");
 
+constexpr int SORT_BITS = 9, SORT_MAX = 1 << SORT_BITS;   // products of a row that is sorted at most
+constexpr int SORT_COLS = (1 << (32 - SORT_BITS)) - 1;    // C's columns up to which it is (32-bit keys)
+constexpr int SORT_NB = 80;                                // blocks of its span from which it is
+
 struct RowArgs {
     int m = 0, k = 0, n = 0, nblk = 0;
     const long long *rpA = nullptr, *rpB = nullptr;
     const int *colA = nullptr, *colB = nullptr;
     const double *valA = nullptr, *valB = nullptr;
+    int sort_max = 0;                         // rows of so many products at most are sorted (0: none)
     float each = 32;                          // light rows: products of an A entry from which an item is a CTA's
     const int2 *rng = nullptr;                // each row of C: its blocks [x, y)
     // The cut table, k rows of width + 1 blocks; null when every row is one
@@ -82,14 +87,18 @@ struct RowArgs {
 };
 
 // What row_products finds (zeroed before).
+constexpr unsigned SEEN_BAD = 1;     // a column of A outside B's rows
+constexpr unsigned SEEN_CUTS = 2;    // a row needs the cut table (more than one item or window)
+constexpr unsigned SEEN_SORT = 4;    // rows of up to 128 (<< 1: 256, << 2: SORT_MAX) products to sort
+
 struct RowStat {
     unsigned long long products, items;       // intermediate products; an upper bound of the items
     unsigned heavy[HEAVY_CLASSES];
     int width;                                // blocks of the widest row
-    int cuts;                                 // a row needs the cut table (more than one item or window)
-    int bad;                                  // a column of A outside B's rows
+    unsigned seen;                            // SEEN_*
     unsigned bitblk;                          // row_symbolic: blocks of kept bitmaps handed out
-    unsigned long long blocks;                // blocks of all rows
+    int pad;
+    unsigned long long blocks;                // blocks of the rows that keep their bitmaps
     unsigned nitems[ITEM_CLASSES];            // row_symbolic: items of each class
 };
 
@@ -99,10 +108,10 @@ cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long lon
 cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat);
 cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut);
 // items: ITEM_CLASSES lists of cap
-cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const unsigned *nheavy,
-                         int width, int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
+cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const RowStat &h,
+                         int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
                          cudaEvent_t fork, cudaEvent_t join);
-cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int4 *items, unsigned cap, const unsigned *n,
+cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int *prod, const int4 *items, unsigned cap, const RowStat &h,
                         const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
                         cudaEvent_t fork, cudaEvent_t join);
 
