@@ -55,6 +55,7 @@ def _cases():
                          _rows(60, 120007, [1, 31, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 0], 23), "AB"),
         "sort_batches": (_rows(150, 300, [64, 33, 32, 65, 130, 7], 24), _rows(300, 100003, [0, 4, 8, 3, 1], 25), "AB"),
         "sort_repeats": (_rows(200, 50, [4, 3, 1, 5], 26), _spread(_rows(50, 150, [128, 40, 100], 27), 900), "AB"),
+        "wide_a": (_rows(20, 9000, [5000, 2049, 2048, 10, 0, 8999], 28), _rows(9000, 3000, [3, 0, 1], 29), "AB"),
         "rmat9": (M.rmat(9, 8, seed=3), None, "AAT"),
         "rmat12": (M.rmat(12, 8, seed=4), None, "AA"),
         "stencil": (M.stencil_27(11, seed=2), None, "AAT"),

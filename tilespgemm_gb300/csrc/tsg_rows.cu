@@ -82,82 +82,144 @@ k_row_sample(RowArgs g, int step, unsigned long long *out)
     if ((threadIdx.x & 31) == 0 && p) atomicAdd(out, (unsigned long long)(p * step));
 }
 
-// Per row of B its first and last block of columns (one thread each).
-__global__ void k_row_extents(const long long *__restrict__ rpB, const int *__restrict__ colB, int kB, int2 *ext)
+// Per row of B its first and last block of columns and its entries (one thread each).
+__global__ void k_row_extents(const long long *__restrict__ rpB, const int *__restrict__ colB, int kB, int4 *ext)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= kB) return;
     const long long s = rpB[k], e = rpB[k + 1];
-    ext[k] = e > s ? make_int2(colB[s] >> ROW_BLK_LOG, colB[e - 1] >> ROW_BLK_LOG) : make_int2(INT_MAX, -1);
+    ext[k] = e > s ? make_int4(colB[s] >> ROW_BLK_LOG, colB[e - 1] >> ROW_BLK_LOG, (int)(e - s), 0)
+                   : make_int4(INT_MAX, -1, 0, 0);
 }
 
-// Per row of C (one warp each): its products, INT_MAX at most, and its blocks
-// [x, y); rows of more than ROW_HEAVY products are listed by weight.
-__global__ void __launch_bounds__(256)
-k_row_products(RowArgs g, const int2 *__restrict__ ext, int *prod, int2 *rng, int *heavy, RowStat *stat)
+// Per row of C its products, INT_MAX at most, and its blocks [x, y); rows of
+// more than ROW_HEAVY products are listed by weight.  One warp a row, four
+// gathers a lane in flight; a row of A longer than WIDE_A entries is left to
+// the whole CTA, whose chain is eight times shorter.  Bound by the latency of
+// a row's chain (row pointer, column, extent); what all rows add up goes
+// through registers and one set of atomics a CTA, of which there are as many
+// as the SMs hold: a flag tested per row is one L2 line for all of them.
+// Measured on GB300 (cold, a launch): uniform, 16 entries a row, 120,007 rows
+// 147 -> 40 us; R-MAT 2^12 x 8 40 -> 8, 2^15 x 16 98 -> 31, 2^18 x 16 406 -> 150.
+constexpr int WIDE_A = 2048, WIDE_LIST = 32;
+
+struct RowSum {
+    long long p = 0;
+    int lo = INT_MAX, hi = -1;
+    bool out = false;
+};
+
+// Entries e, e + stride, ... of A's row up to e1, four in flight.
+__device__ __forceinline__ RowSum sum_entries(const RowArgs &g, const int4 *__restrict__ ext, long long e, long long e1,
+                                              int stride)
 {
-    __shared__ unsigned long long s_p[8], s_i[8], s_b[8];
-    __shared__ int s_w[8];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned long long sp = 0, si = 0, sb = 0;
-    int width = 0;
-    for (long long r = blockIdx.x * 8ll + warp; r < g.m; r += gridDim.x * 8ll) {
-        long long p = 0;
-        int lo = INT_MAX, hi = -1;
-        bool out = false;
-        const long long e1 = g.rpA[r + 1];
-        for (long long e = g.rpA[r] + lane; e < e1; e += 128) {
-            int k[4];
+    RowSum s;
+    for (; e < e1; e += 4 * stride) {
+        int k[4];
+        int4 x[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) k[u] = e + 32 * u < e1 ? g.colA[e + 32 * u] : -1;
+        for (int u = 0; u < 4; ++u) k[u] = e + u * stride < e1 ? g.colA[e + u * stride] : -1;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if ((unsigned)k[u] < (unsigned)g.k) {
-                    p += g.rpB[k[u] + 1] - g.rpB[k[u]];
-                    const int2 x = ext[k[u]];
-                    lo = min(lo, x.x);
-                    hi = max(hi, x.y);
-                } else if (e + 32 * u < e1) {
-                    out = true;
-                }
-            }
-        }
-        p = warp_sum_ll(p);
-        lo = __reduce_min_sync(FULL, lo);
-        hi = __reduce_max_sync(FULL, hi);
-        out = __any_sync(FULL, out);
-        if (lane == 0) {
-            unsigned seen = 0;
-            sp += (unsigned long long)p;
-            prod[r] = (int)min(p, (long long)INT_MAX);
-            const int nb = hi < lo ? 0 : hi - lo + 1;
-            rng[r] = make_int2(nb ? lo : 0, nb ? hi + 1 : 0);
-            if (sorted_row(g, p, nb)) {          // no bitmap, no item
-                seen = p > 256 ? SEEN_SORT << 2 : p > 128 ? SEEN_SORT << 1 : SEEN_SORT;
-            } else {
-                width = max(width, nb);
-                if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
-                si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
-                if (p > LIGHT_ROW || nb > SYM_BLKS) seen = SEEN_CUTS;
-            }
-            if (out) seen |= SEEN_BAD;
-            if (seen & ~*(volatile unsigned *)&stat->seen) atomicOr(&stat->seen, seen);
-            if (p > ROW_HEAVY) {
-                const int c = heavy_class(p);
-                heavy[(long long)c * g.m + atomicAdd(stat->heavy + c, 1u)] = (int)r;
-            }
+        for (int u = 0; u < 4; ++u)
+            x[u] = (unsigned)k[u] < (unsigned)g.k ? ext[k[u]] : make_int4(INT_MAX, -1, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            s.lo = min(s.lo, x[u].x);
+            s.hi = max(s.hi, x[u].y);
+            s.p += x[u].z;
+            s.out |= e + u * stride < e1 && (unsigned)k[u] >= (unsigned)g.k;
         }
     }
-    if (lane == 0) { s_p[warp] = sp; s_i[warp] = si; s_b[warp] = sb; s_w[warp] = width; }
+    s.p = warp_sum_ll(s.p);
+    s.lo = __reduce_min_sync(FULL, s.lo);
+    s.hi = __reduce_max_sync(FULL, s.hi);
+    s.out = __any_sync(FULL, s.out);
+    return s;
+}
+
+__global__ void __launch_bounds__(256)
+k_row_products(RowArgs g, const int4 *__restrict__ ext, int *prod, int2 *rng, int *heavy, RowStat *stat)
+{
+    __shared__ unsigned long long s_p[8], s_i[8], s_b[8];
+    __shared__ int s_w[8], s_lo[8], s_hi[8], s_long[WIDE_LIST], s_nlong;
+    __shared__ long long s_sum[8];
+    __shared__ unsigned s_seen;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) s_nlong = 0, s_seen = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    unsigned long long sp = 0, si = 0, sb = 0;
+    unsigned seen = 0;
+    int width = 0;
+    auto finish = [&](int r, const RowSum &s) {      // one thread
+        const long long p = s.p;
+        const int nb = s.hi < s.lo ? 0 : s.hi - s.lo + 1;
+        prod[r] = (int)min(p, (long long)INT_MAX);
+        rng[r] = make_int2(nb ? s.lo : 0, nb ? s.hi + 1 : 0);
+        sp += (unsigned long long)p;
+        if (sorted_row(g, p, nb)) {          // no bitmap, no item
+            seen |= p > 256 ? SEEN_SORT << 2 : p > 128 ? SEEN_SORT << 1 : SEEN_SORT;
+        } else {
+            width = max(width, nb);
+            if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
+            si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
+            if (p > LIGHT_ROW || nb > SYM_BLKS) seen |= SEEN_CUTS;
+        }
+        if (s.out) seen |= SEEN_BAD;
+        if (p > ROW_HEAVY) {
+            const int c = heavy_class(p);
+            heavy[(long long)c * g.m + atomicAdd(stat->heavy + c, 1u)] = r;
+        }
+    };
+    for (long long r = blockIdx.x * 8ll + warp; r < g.m; r += gridDim.x * 8ll) {
+        const long long e0 = g.rpA[r], e1 = g.rpA[r + 1];
+        if (e1 - e0 > WIDE_A) {
+            int at = WIDE_LIST;
+            if (lane == 0) at = atomicAdd(&s_nlong, 1);
+            at = __shfl_sync(FULL, at, 0);
+            if (at < WIDE_LIST) {
+                if (lane == 0) s_long[at] = (int)r;
+                continue;
+            }
+        }
+        const RowSum s = sum_entries(g, ext, e0 + lane, e1, 32);
+        if (lane == 0) finish((int)r, s);
+    }
+    __syncthreads();
+    const int nlong = min(s_nlong, WIDE_LIST);
+    for (int t = 0; t < nlong; ++t) {
+        const int r = s_long[t];
+        RowSum s = sum_entries(g, ext, g.rpA[r] + tid, g.rpA[r + 1], 256);
+        if (lane == 0) {
+            s_sum[warp] = s.p;
+            s_lo[warp] = s.lo;
+            s_hi[warp] = s.out ? INT_MIN : s.hi;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            for (int q = 1; q < 8; ++q) {
+                s.p += s_sum[q];
+                s.lo = min(s.lo, s_lo[q]);
+                s.out |= s_hi[q] == INT_MIN;
+                s.hi = max(s.hi, s_hi[q]);
+            }
+            finish(r, s);
+        }
+        __syncthreads();
+    }
+    if (lane == 0) {
+        s_p[warp] = sp; s_i[warp] = si; s_b[warp] = sb; s_w[warp] = width;
+        if (seen) atomicOr(&s_seen, seen);
+    }
+    __syncthreads();
+    if (tid == 0) {
         unsigned long long a = 0, b = 0, c = 0;
         int w = 0;
         for (int q = 0; q < 8; ++q) { a += s_p[q]; b += s_i[q]; c += s_b[q]; w = max(w, s_w[q]); }
         atomicAdd(&stat->products, a);
         atomicAdd(&stat->items, b);
-        atomicAdd(&stat->blocks, c);
-        if (w > *(volatile int *)&stat->width) atomicMax(&stat->width, w);
+        if (c) atomicAdd(&stat->blocks, c);
+        if (w) atomicMax(&stat->width, w);
+        if (s_seen) atomicOr(&stat->seen, s_seen);
     }
 }
 
@@ -695,7 +757,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
 // Bound by issue (the network: 650 instructions for 256 keys); the bitmap of
 // such a row took 3,000 over 98 blocks, and 27 KB of shared memory.
 // Measured on GB300: uniform 120,007 x 80,021 x 100,003, 192 products a row over
-// 98 blocks: 2,080 -> 727 us a call (k_row_sort 140 us to count, 227 to fill).
+// 98 blocks: 2,080 -> 650 us a call (k_row_sort 140 us to count, 227 to fill).
 constexpr int SORT_WARPS = 4;
 
 struct __align__(16) Share {     // one A entry's B row: entry f + delta for the row's product f
@@ -915,7 +977,7 @@ cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long lon
 
 cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat)
 {
-    int2 *ext = pool.alloc_n<int2>(g.k);
+    int4 *ext = pool.alloc_n<int4>(g.k);
     if (!ext) return pool.err;
     k_row_extents<<<(unsigned)((g.k + 255) / 256), 256, 0, pool.stream>>>(g.rpB, g.colB, g.k, ext);
     k_row_products<<<warps_grid(g.m), 256, 0, pool.stream>>>(g, ext, prod, rng, heavy, stat);
