@@ -160,6 +160,8 @@ struct tsg_ctx {
     bool counted = false;            // entered in the pinned cache's count of live contexts
     cudaStream_t side = nullptr;     // second stream for kernels that overlap the main one's (fork/join by events)
     cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t lane[ROW_LANES - 1] = {};       // the row path's, with side
+    cudaEvent_t lane_join[ROW_LANES - 1] = {};
     // host-link copies beside the kernels: operand values up during the
     // symbolic phase, C's row pointers and column indices down during the
     // numeric step
@@ -1000,6 +1002,12 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     P.rowptrC = P.own<long long>(pool, P.m + 1);
     if (!prod || !heavy || !rowcnt || !rng || !P.rowptrC) return fail(TSG_ERR_OOM, "device pool allocation failed (row path)");
     g.rng = rng;
+    RowLanes lanes;
+    lanes.fork = ctx->fork;
+    for (int t = 0; t < ROW_LANES; ++t) {
+        lanes.lane[t] = t == 0 ? ctx->side : ctx->lane[t - 1];
+        lanes.join[t] = t == 0 ? ctx->join : ctx->lane_join[t - 1];
+    }
     CUDA_OK(row_products(pool, g, prod, rng, heavy, rs));
     tsg_status r = host_wait(ctx, &P.nsync);
     if (r) return r;
@@ -1038,8 +1046,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
         }
         cudaGetLastError();
     }
-    CUDA_OK(row_symbolic(pool, g, prod, heavy, h, rowcnt, items, (unsigned)cap, rs, ctx->side,
-                         ctx->fork, ctx->join));
+    CUDA_OK(row_symbolic(pool, g, prod, heavy, h, rowcnt, items, (unsigned)cap, rs, lanes));
     CUDA_OK(scan_i32_to_i64(pool, rowcnt, P.rowptrC, P.m, ctx->dflags));
     CUDA_OK(cudaMemcpyAsync(ctx->dstat + ST_NNZC, P.rowptrC + P.m, sizeof(long long), cudaMemcpyDeviceToDevice,
                             ctx->stream));
@@ -1055,8 +1062,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     val = pool.out_n<double>(P.nnzC);
     if (!col || !val) return fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
     P.wait_values(ctx->stream);
-    CUDA_OK(row_numeric(pool, g, prod, items, (unsigned)cap, h, P.rowptrC, col, val, ctx->dflags, ctx->side,
-                        ctx->fork, ctx->join));
+    CUDA_OK(row_numeric(pool, g, prod, items, (unsigned)cap, h, P.rowptrC, col, val, ctx->dflags, lanes));
     taken = true;
     return TSG_OK;
 }
@@ -1470,6 +1476,10 @@ tsg_status tsg_create(tsg_ctx **out, int device, const tsg_opts *opts)
         cudaEventCreateWithFlags(&c->copy_done, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ext_ev, cudaEventDisableTiming) != cudaSuccess)
         return cleanup(fail(TSG_ERR_CUDA, "cudaEventCreate failed"));
+    for (int t = 0; t < ROW_LANES - 1; ++t)
+        if (cudaStreamCreateWithFlags(&c->lane[t], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&c->lane_join[t], cudaEventDisableTiming) != cudaSuccess)
+            return cleanup(fail(TSG_ERR_CUDA, "cudaStreamCreate failed"));
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.handleTypes = cudaMemHandleTypeNone;
@@ -1507,6 +1517,8 @@ tsg_status tsg_destroy(tsg_ctx *c)
     if (c->fork) cudaEventDestroy(c->fork);
     if (c->join) cudaEventDestroy(c->join);
     if (c->side) { cudaStreamSynchronize(c->side); cudaStreamDestroy(c->side); }
+    for (auto &l : c->lane) if (l) { cudaStreamSynchronize(l); cudaStreamDestroy(l); }
+    for (auto &e : c->lane_join) if (e) cudaEventDestroy(e);
     if (c->copy) { cudaStreamSynchronize(c->copy); cudaStreamDestroy(c->copy); }
     for (cudaEvent_t e : {c->cfork, c->vals_ev, c->cols_ev, c->copy_done, c->ext_ev}) if (e) cudaEventDestroy(e);
     for (auto &sh : c->small_shapes) if (sh.rowptr) cudaFreeAsync(sh.rowptr, c->stream);

@@ -942,6 +942,24 @@ size_t sym_smem(int width) { return (size_t)std::min(width, SYM_BLKS) * (ROW_BLK
 
 unsigned warps_grid(long long rows) { return (unsigned)std::min<long long>(std::max<long long>((rows + 7) / 8, 1), 152 * 32); }
 
+cudaError_t fork_lanes(cudaStream_t s, const RowLanes &l, int n)
+{
+    cudaError_t e = n > 0 ? cudaEventRecord(l.fork, s) : cudaSuccess;
+    for (int t = 0; t < n && e == cudaSuccess; ++t) e = cudaStreamWaitEvent(l.lane[t], l.fork, 0);
+    return e;
+}
+
+cudaError_t join_lanes(cudaStream_t s, const RowLanes &l, int n)
+{
+    cudaError_t e = cudaSuccess;
+    for (int t = 0; t < n; ++t) {      // every lane, also after a failure
+        cudaError_t j = cudaEventRecord(l.join[t], l.lane[t]);
+        if (j == cudaSuccess) j = cudaStreamWaitEvent(s, l.join[t], 0);
+        if (e == cudaSuccess) e = j;
+    }
+    return e;
+}
+
 template <int NT>
 cudaError_t numeric_class(cudaStream_t s, const RowArgs &g, const int4 *items, long long n, int c,
                           const long long *rowptrC, int *colC, double *valC, int *flags)
@@ -995,8 +1013,7 @@ cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut)
 }
 
 cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const RowStat &hs,
-                         int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
-                         cudaEvent_t fork, cudaEvent_t join)
+                         int *rowcnt, int4 *items, unsigned cap, RowStat *stat, const RowLanes &l)
 {
     cudaStream_t s = pool.stream;
     const int width = hs.width;
@@ -1004,51 +1021,55 @@ cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const in
     HeavyRows h;
     int total = 0;
     for (int c = 0; c < HEAVY_CLASSES; ++c) total += h.n[c] = (int)hs.heavy[c];
-    cudaError_t e = cudaEventRecord(fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+    cudaError_t e = cudaSuccess;
+    if (width == 0)      // every row is sorted, or empty
+        e = cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)g.m, s);
+    const bool sorts = hs.seen & SEEN_SORT * 7;
+    const int lanes = sorts ? 3 : 2;
+    if (e == cudaSuccess) e = fork_lanes(s, l, lanes);
     if (e != cudaSuccess) return e;
     if (total > 0) {   // the heaviest first: the others run beside their tail
         HeavyRows hl = h;
         hl.list = heavy;
         hl.m = g.m;
-        k_row_symbolic<1024><<<(unsigned)total, 1024, sm, side>>>(g, prod, ROW_HEAVY, INT_MAX, hl, width, rowcnt, items, cap, stat);
+        k_row_symbolic<1024><<<(unsigned)total, 1024, sm, l.lane[0]>>>(g, prod, ROW_HEAVY, INT_MAX, hl, width, rowcnt, items, cap, stat);
         ::tsg::count_launch();
     }
     if (width > 0) {
         k_row_symbolic<256><<<(unsigned)g.m, 256, sm, s>>>(g, prod, ROW_TINY, ROW_HEAVY, h, width, rowcnt, items, cap, stat);
-        k_row_symbolic<64><<<(unsigned)g.m, 64, sm, side>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, stat);
+        k_row_symbolic<64><<<(unsigned)g.m, 64, sm, l.lane[1]>>>(g, prod, 0, ROW_TINY, h, width, rowcnt, items, cap, stat);
         ::tsg::count_launch();
         ::tsg::count_launch();
-    } else {      // every row is sorted, or empty
-        e = cudaMemsetAsync(rowcnt, 0, sizeof(int) * (size_t)g.m, s);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = sort_rows<false>(s, g, prod, hs, rowcnt, nullptr, nullptr, nullptr, nullptr);
-    cudaError_t j = cudaEventRecord(join, side);
-    if (j == cudaSuccess) j = cudaStreamWaitEvent(s, join, 0);
+    if (e == cudaSuccess) e = sort_rows<false>(l.lane[2], g, prod, hs, rowcnt, nullptr, nullptr, nullptr, nullptr);
+    const cudaError_t j = join_lanes(s, l, lanes);
     return e == cudaSuccess ? j : e;
 }
 
 cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int *prod, const int4 *items, unsigned cap, const RowStat &h,
-                        const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
-                        cudaEvent_t fork, cudaEvent_t join)
+                        const long long *rowptrC, int *colC, double *valC, int *flags, const RowLanes &l)
 {
     cudaStream_t s = pool.stream;
-    cudaError_t e = cudaEventRecord(fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
-    // two streams, the longest chains first on each: a class's last items run
-    // beside the next ones
-    constexpr int order[ITEM_CLASSES] = {3, 2, 1, 0, 4, 5, 6};
-    for (int q = 0; q < ITEM_CLASSES && e == cudaSuccess; ++q) {
-        const int c = order[q];
-        cudaStream_t on = q % 2 ? s : side;
-        const int4 *list = items + (long long)c * cap;
-        e = c < CLASS_WARP ? numeric_class<32>(on, g, list, h.nitems[c], c, rowptrC, colC, valC, flags)
-                           : numeric_class<NT_WIDE>(on, g, list, h.nitems[c], c, rowptrC, colC, valC, flags);
+    // every class on a stream of its own, so that none waits for another's last
+    // items, and in this order, the longest chains (large items, and a heavy
+    // row's many small ones) first.  Two streams in place of these: R-MAT
+    // 2^15 x 16 A*A^T 2,190 us a call for 1,692, 2^16 x 12 A*A 2,950 for 2,552
+    constexpr int order[ITEM_CLASSES] = {3, 2, 0, 1, 6, 5, 4};
+    static_assert(ROW_LANES == ITEM_CLASSES - 1, "a stream for each class");
+    int list[ITEM_CLASSES], n = 0;
+    for (int c : order)
+        if (h.nitems[c] > 0) list[n++] = c;
+    cudaError_t e = fork_lanes(s, l, n - 1);
+    for (int q = 0; q < n && e == cudaSuccess; ++q) {
+        const int c = list[q];
+        cudaStream_t on = q == n - 1 ? s : l.lane[q];
+        const int4 *it = items + (long long)c * cap;
+        e = c < CLASS_WARP ? numeric_class<32>(on, g, it, h.nitems[c], c, rowptrC, colC, valC, flags)
+                           : numeric_class<NT_WIDE>(on, g, it, h.nitems[c], c, rowptrC, colC, valC, flags);
     }
     if (e == cudaSuccess) e = sort_rows<true>(s, g, prod, h, nullptr, rowptrC, colC, valC, flags);
-    cudaError_t j = cudaEventRecord(join, side);
-    if (j == cudaSuccess) j = cudaStreamWaitEvent(s, join, 0);
+    const cudaError_t j = join_lanes(s, l, n - 1);
     return e == cudaSuccess ? j : e;
 }
 

@@ -102,6 +102,13 @@ struct RowStat {
     unsigned nitems[ITEM_CLASSES];            // row_symbolic: items of each class
 };
 
+// Streams beside the main one; fork and join tie them to it.
+constexpr int ROW_LANES = ITEM_CLASSES - 1;
+struct RowLanes {
+    cudaStream_t lane[ROW_LANES];
+    cudaEvent_t fork, join[ROW_LANES];
+};
+
 cudaError_t rows_init_attributes();
 // adds step * the products of every step-th row
 cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out);
@@ -109,10 +116,8 @@ cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int
 cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut);
 // items: ITEM_CLASSES lists of cap
 cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const RowStat &h,
-                         int *rowcnt, int4 *items, unsigned cap, RowStat *stat, cudaStream_t side,
-                         cudaEvent_t fork, cudaEvent_t join);
+                         int *rowcnt, int4 *items, unsigned cap, RowStat *stat, const RowLanes &l);
 cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int *prod, const int4 *items, unsigned cap, const RowStat &h,
-                        const long long *rowptrC, int *colC, double *valC, int *flags, cudaStream_t side,
-                        cudaEvent_t fork, cudaEvent_t join);
+                        const long long *rowptrC, int *colC, double *valC, int *flags, const RowLanes &l);
 
 }  // namespace tsg
