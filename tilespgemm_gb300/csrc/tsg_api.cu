@@ -1054,8 +1054,8 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     if (r) return r;
     P.nnzC = ctx->hstat[ST_NNZC];
     memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
-    for (unsigned n : h.nitems)
-        if (n > cap) return fail(TSG_ERR_CUDA, "internal: the row path's items outgrew their bound");
+    for (int c = 0; c < ITEM_CLASSES; ++c)
+        if ((long long)h.front[c] + h.back[c] > cap) return fail(TSG_ERR_CUDA, "internal: the row path's items outgrew their bound");
     if (!batch && output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))
         return fail(TSG_ERR_INT32_OVERFLOW, "C has %lld entries; int32 row pointers cannot hold them", P.nnzC);
     col = pool.out_n<int>(P.nnzC);

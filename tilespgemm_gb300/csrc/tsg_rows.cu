@@ -267,7 +267,6 @@ __global__ void __launch_bounds__(NT)
 k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRows heavy, int width, int *rowcnt,
                int4 *items, unsigned cap, RowStat *stat)
 {
-    unsigned *nitems = stat->nitems;
     __shared__ unsigned s_bit;
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned s_sym[];
@@ -385,13 +384,18 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
     // written where the row's share of the class's list begins.
     __shared__ unsigned s_cls[ITEM_CLASSES];
     const long long la = a1 - a0;
+    const bool early = la > LONG_A;
+    unsigned *nitems = early ? stat->front : stat->back;
+    auto put = [&](int c, unsigned i, int4 it) {
+        if (i < cap) items[(unsigned long long)c * cap + (early ? i : cap - 1 - i)] = it;
+    };
     int tclose = ITEM_T, bmax = ITEM_BLKS;      // a row's items close at so many entries, or blocks
     auto close = [&](int j, int e, int pj, int pe, bool write) {   // blocks [pj, j), entries [pe, e) of the row
         const int z = e - pe, nb = j - pj;
         if (z <= 0) return;
         const int c = item_class(z, nb, tclose == ITEM_T || (float)p * (float)z <= g.each * (float)la * (float)cnt[nblk]);
         const unsigned i = atomicAdd(s_cls + c, 1u);
-        if (write && i < cap) items[(unsigned long long)c * cap + i] = make_int4(r, first + pj, pe, (nb << 16) | z);
+        if (write) put(c, i, make_int4(r, first + pj, pe, (nb << 16) | z));
     };
     auto pass = [&](bool write) -> int {
         int run = 0, pj = 0, pe = 0;
@@ -434,7 +438,7 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
         if (lane == 0 && z > 0) {
             const int c = item_class(z, nblk, (float)p <= g.each * (float)la);
             const unsigned i = atomicAdd(nitems + c, 1u);
-            if (i < cap) items[(unsigned long long)c * cap + i] = make_int4(r, first, 0, (nblk << 16) | z);
+            put(c, i, make_int4(r, first, 0, (nblk << 16) | z));
         }
         return;
     }
@@ -461,7 +465,7 @@ struct __align__(16) Step {  // up to NT of one A entry's products: B's entries 
 // themselves; warps without a product only meet the barrier.
 template <int NT>
 __global__ void __launch_bounds__(NT)
-k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__restrict__ rowptrC,
+k_row_numeric(RowArgs g, const int4 *__restrict__ items, unsigned front, unsigned last, const long long *__restrict__ rowptrC,
               int *__restrict__ colC, double *__restrict__ valC, int *flags)
 {
     constexpr int NW = NT / 32, STEPS = row_steps(NT);
@@ -469,7 +473,7 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, const long long *__rest
     __shared__ int s_sum[NW + 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto sync = [] { if constexpr (NT > 32) __syncthreads(); else __syncwarp(); };
-    const int4 it = items[blockIdx.x];
+    const int4 it = items[blockIdx.x < front ? blockIdx.x : last - blockIdx.x];
     const int r = it.x, j0 = it.y, z = it.w & 0xffff, nb = it.w >> 16;
     const int c0 = j0 << ROW_BLK_LOG, nw = nb * (ROW_BLK / 32);
     const bool dense = item_dense(z, nb);
@@ -961,11 +965,12 @@ cudaError_t join_lanes(cudaStream_t s, const RowLanes &l, int n)
 }
 
 template <int NT>
-cudaError_t numeric_class(cudaStream_t s, const RowArgs &g, const int4 *items, long long n, int c,
-                          const long long *rowptrC, int *colC, double *valC, int *flags)
+cudaError_t numeric_class(cudaStream_t s, const RowArgs &g, const int4 *items, unsigned cap, const RowStat &h,
+                          int c, const long long *rowptrC, int *colC, double *valC, int *flags)
 {
-    if (n <= 0) return cudaSuccess;
-    k_row_numeric<NT><<<(unsigned)n, NT, class_smem(c) + row_steps(NT) * sizeof(Step), s>>>(g, items, rowptrC, colC, valC, flags);
+    const unsigned n = h.front[c] + h.back[c];
+    k_row_numeric<NT><<<n, NT, class_smem(c) + row_steps(NT) * sizeof(Step), s>>>(
+        g, items, h.front[c], cap - 1 + h.front[c], rowptrC, colC, valC, flags);
     ::tsg::count_launch();
     return cudaGetLastError();
 }
@@ -1059,14 +1064,14 @@ cudaError_t row_numeric(Pool &pool, const RowArgs &g, const int *prod, const int
     static_assert(ROW_LANES == ITEM_CLASSES - 1, "a stream for each class");
     int list[ITEM_CLASSES], n = 0;
     for (int c : order)
-        if (h.nitems[c] > 0) list[n++] = c;
+        if (h.front[c] + h.back[c] > 0) list[n++] = c;
     cudaError_t e = fork_lanes(s, l, n - 1);
     for (int q = 0; q < n && e == cudaSuccess; ++q) {
         const int c = list[q];
         cudaStream_t on = q == n - 1 ? s : l.lane[q];
         const int4 *it = items + (long long)c * cap;
-        e = c < CLASS_WARP ? numeric_class<32>(on, g, it, h.nitems[c], c, rowptrC, colC, valC, flags)
-                           : numeric_class<NT_WIDE>(on, g, it, h.nitems[c], c, rowptrC, colC, valC, flags);
+        e = c < CLASS_WARP ? numeric_class<32>(on, g, it, cap, h, c, rowptrC, colC, valC, flags)
+                           : numeric_class<NT_WIDE>(on, g, it, cap, h, c, rowptrC, colC, valC, flags);
     }
     if (e == cudaSuccess) e = sort_rows<true>(s, g, prod, h, nullptr, rowptrC, colC, valC, flags);
     const cudaError_t j = join_lanes(s, l, n - 1);

@@ -33,6 +33,11 @@ __host__ __device__ constexpr int row_steps(int nt) { return nt > 32 ? 128 : 32;
 // and 2 items of NT_WIDE threads; the occupancy hides their loads (one class
 // of 20 KB in place of the first two: R-MAT 2^18 A*A^T 52.3 against 45.3 ms).
 constexpr int ITEM_CLASSES = 7, CLASS_WARP = 4;
+// A row's items are chains over its A entries.  Those of rows with more than
+// LONG_A start first, or they run on alone at the end (R-MAT 2^15 x 16 A*A^T
+// 1,692 us a call in any order, 1,494 so, and 1,515 to 1,545 from 128 to 2,048;
+// 2^12 x 8 414 and 395).
+constexpr int LONG_A = 256;
 __host__ __device__ constexpr int class_smem(int c)
 {
     return c == 0 ? 9 << 10 : c == 1 ? 14 << 10 : c == 2 ? 20 << 10 : c == 3 ? 34 << 10 : c == 4 ? 40 << 10 : c == 5 ? 72 << 10 : 112 << 10;
@@ -99,7 +104,9 @@ struct RowStat {
     unsigned bitblk;                          // row_symbolic: blocks of kept bitmaps handed out
     int pad;
     unsigned long long blocks;                // blocks of the rows that keep their bitmaps
-    unsigned nitems[ITEM_CLASSES];            // row_symbolic: items of each class
+    // row_symbolic: items of each class; those of rows with many A entries, the
+    // long chains, fill its list from the front, the others from the back
+    unsigned front[ITEM_CLASSES], back[ITEM_CLASSES];
 };
 
 // Streams beside the main one; fork and join tie them to it.
