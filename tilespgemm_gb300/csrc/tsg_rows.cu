@@ -753,15 +753,17 @@ k_row_numeric(RowArgs g, const int4 *__restrict__ items, unsigned front, unsigne
 
 // ---- rows of few products: sorted in registers ---------------------------------
 //
-// A row of up to SORT_MAX products needs no bitmap of its span: one warp
-// sorts the keys (column, product) -- E a lane, a bitonic network, strides
-// below E inside a lane -- and a column's products then lie side by side in
-// product order: counted for C's row, or applied to its entry in that order.
-// The product number in the low bits leaves 23 bits for the column.
+// A row of up to SORT_MAX products needs no bitmap of its span.  To count its
+// columns one warp puts them in a hash table, half full at most; to fill C's
+// row it sorts the keys (column, product) -- E a lane, a bitonic network,
+// strides below E inside a lane -- and a column's products then lie side by
+// side in product order, to be applied to its entry in that order.  The
+// product number in the low bits leaves 23 bits for the column.
 // Bound by issue (the network: 650 instructions for 256 keys); the bitmap of
 // such a row took 3,000 over 98 blocks, and 27 KB of shared memory.
 // Measured on GB300: uniform 120,007 x 80,021 x 100,003, 192 products a row over
-// 98 blocks: 2,080 -> 650 us a call (k_row_sort 140 us to count, 227 to fill).
+// 98 blocks: 2,080 -> 600 us a call (k_row_sort 104 us to count, 140 when it
+// sorted there too, and 227 to fill).
 constexpr int SORT_WARPS = 4;
 
 struct __align__(16) Share {     // one A entry's B row: entry f + delta for the row's product f
@@ -771,7 +773,7 @@ struct __align__(16) Share {     // one A entry's B row: entry f + delta for the
 
 template <int E, bool FILL>
 struct SortSmem {
-    unsigned key[32 * E];
+    unsigned met[64 * E];           // the columns met: a hash table, half full at most
     Share share[32];
 };
 template <int E>
@@ -842,7 +844,13 @@ k_row_sort(RowArgs g, const int *__restrict__ prod, int lo, int *rowcnt, const l
     const int2 rng = g.rng[r];
     if (!sorted_row(g, p, rng.y - rng.x)) return;
     SortSmem<E, FILL> &w = s_w[warp];
-    for (int t = p + lane; t < 32 * E; t += 32) w.key[t] = 0xffffffffu;
+    if constexpr (FILL) {
+        for (int t = p + lane; t < 32 * E; t += 32) w.key[t] = 0xffffffffu;
+    } else {
+        for (int t = lane; t < 16 * E; t += 32)
+            reinterpret_cast<uint4 *>(w.met)[t] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    }
+    int fresh = 0;
     const long long a1 = g.rpA[r + 1];
     int f0 = 0;                                     // products before this batch of A entries
     for (long long a = g.rpA[r]; a < a1; a += 32) {
@@ -873,31 +881,40 @@ k_row_sort(RowArgs g, const int *__restrict__ prod, int lo, int *rowcnt, const l
             const int f = base + lane;
             if (f < T) {
                 const int e = w.share[q].delta + f;
-                w.key[f0 + f] = (unsigned)g.colB[e] << SORT_BITS | (unsigned)(f0 + f);
-                if constexpr (FILL) w.ab[f0 + f] = make_double2(w.share[q].a, g.valB[e]);
+                const unsigned c = (unsigned)g.colB[e];
+                if constexpr (FILL) {
+                    w.key[f0 + f] = c << SORT_BITS | (unsigned)(f0 + f);
+                    w.ab[f0 + f] = make_double2(w.share[q].a, g.valB[e]);
+                } else {
+                    unsigned h = (c * 0x9e3779b1u) >> (32 - __ffs(64 * E) + 1);
+                    unsigned was;
+                    while ((was = atomicCAS(&w.met[h], ~0u, c)) != ~0u && was != c) h = (h + 1) & (64 * E - 1);
+                    fresh += was == ~0u;
+                }
             }
         }
         f0 += T;
     }
-    __syncwarp();
-    unsigned x[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) x[e] = w.key[lane * E + e];
-    sort_keys<E>(x, lane);
-    // the first product of each column starts an entry of C
-    unsigned before = __shfl_up_sync(FULL, x[E - 1], 1);
-    unsigned heads = 0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const bool first = lane == 0 && e == 0;
-        if (x[e] != 0xffffffffu && (first || (x[e] >> SORT_BITS) != (before >> SORT_BITS))) heads |= 1u << e;
-        before = x[e];
-    }
-    const int n = __popc(heads);
     if constexpr (!FILL) {
-        const int z = (int)__reduce_add_sync(FULL, (unsigned)n);
+        const int z = (int)__reduce_add_sync(FULL, (unsigned)fresh);
         if (lane == 0) rowcnt[r] = z;
+        return;
     } else {
+        __syncwarp();
+        unsigned x[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[e] = w.key[lane * E + e];
+        sort_keys<E>(x, lane);
+        // the first product of each column starts an entry of C
+        unsigned before = __shfl_up_sync(FULL, x[E - 1], 1);
+        unsigned heads = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const bool first = lane == 0 && e == 0;
+            if (x[e] != 0xffffffffu && (first || (x[e] >> SORT_BITS) != (before >> SORT_BITS))) heads |= 1u << e;
+            before = x[e];
+        }
+        const int n = __popc(heads);
         const int incl = warp_incl_scan(n, lane), z = __shfl_sync(FULL, incl, 31);
         int o = incl - n;
 #pragma unroll
