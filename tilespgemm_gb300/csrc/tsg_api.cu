@@ -575,20 +575,54 @@ tsg_status stage_into_plan(tsg_ctx *ctx, Pool &pool, PlanData &P, const tsg_csr 
 // - A row costs the row path a few microseconds of a CTA whatever it holds:
 //   rows of under 128 products go by tiles when there are many (96^3 7-point
 //   stencil, 48 a row: 2.0 ms tiled, 5.2 by rows).
+constexpr long long ROW_PRODUCTS = 24000000;
+constexpr int ROW_FEW = 65536;
 bool rows_pay(const PlanData &P, long long products, long long runsA, long long runsB)
 {
     const bool full = products >= 128ll * P.m;
-    if (products <= 24000000) return full || P.m <= 65536;
+    if (products <= ROW_PRODUCTS) return full || P.m <= ROW_FEW;
     return full && 2 * P.nnzA < 3 * runsA && 2 * P.nnzB < 3 * runsB;
 }
 
 // Symbolic phase: staging, A^T for A*A^T, tiles, step 1, step 2 (two host waits).
 // `keep` = the plan outlives the call (device operands are copied).
-// by_rows (optional): the caller can take the row path; set when the staged
-// operands qualify for it, and then nothing but the staging is done.
+// The row path's start: its per-row arrays and what row_products found.
+struct RowStart {
+    bool take = false;       // the staged operands qualify for the row path
+    bool counted = false;    // row_products ran, its findings are in h
+    int *prod = nullptr, *heavy = nullptr;
+    int2 *rng = nullptr;
+    RowStat h{};
+};
+
+RowArgs row_args(const PlanData &P)
+{
+    RowArgs g;
+    g.m = P.m; g.k = P.k; g.n = P.n; g.nblk = ceil_div_i(P.n, ROW_BLK);
+    g.rpA = P.rpA; g.rpB = P.rpB; g.colA = P.colA; g.colB = P.colB; g.valA = P.valA; g.valB = P.valB;
+    g.width = g.nblk;
+    g.sort_max = P.n <= SORT_COLS ? SORT_MAX : 0;
+    return g;
+}
+
+// Launches row_products; RowStat lands in the bins' slots at the next wait.
+tsg_status row_count(tsg_ctx *ctx, Pool &pool, Scratch &sc, const PlanData &P, RowStart &rs)
+{
+    static_assert(sizeof(RowStat) <= 8 * BS_SLOTS, "the row path's statistics fit the bins' slots");
+    rs.prod = sc.get<int>(P.m);
+    rs.heavy = sc.get<int>((long long)HEAVY_CLASSES * P.m);
+    rs.rng = sc.get<int2>(P.m);
+    if (!rs.prod || !rs.heavy || !rs.rng) return fail(TSG_ERR_OOM, "device pool allocation failed (row path)");
+    CUDA_OK(row_products(pool, row_args(P), rs.prod, rs.rng, rs.heavy, reinterpret_cast<RowStat *>(ctx->dstat + ST_BINS),
+                         ctx->dflags));
+    return TSG_OK;
+}
+
+// rows (optional): the caller can take the row path; rows->take is set when the
+// staged operands qualify for it, and then nothing but the staging is done.
 tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const tsg_csr *A, const tsg_csr *B,
                          PlanData &P, bool keep, bool want_cub, PhaseTimer &tm, bool reset_flags = true,
-                         bool *by_rows = nullptr)
+                         RowStart *rows = nullptr)
 {
     const bool validate = ctx->opts.validate != 0;
     tsg_status r = check_op(op, A, B);
@@ -629,24 +663,32 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
     }
     bool order_known = false;      // B's order is already counted
     long long unsorted = 0;
-    if (by_rows) {
-        *by_rows = false;
+    if (rows) {
+        *rows = RowStart();
         if (P.nnzA > 0 && P.nnzB > 0) {
             // tile runs of A and B, sampled products, and whether B's rows increase, decide
             unsigned long long *rs = reinterpret_cast<unsigned long long *>(ctx->dstat);
             if (op != TSG_OP_AA)
                 CUDA_OK(aux_rows_increasing(pool, P.rpA, P.colA, P.m, P.k, P.nnzA, rs + ST_NNZCUB, rs + ST_TILESA));
             CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.n, P.nnzB, rs + ST_BUNSORTED, rs + ST_TILESB));
-            RowArgs g;
-            g.m = P.m; g.k = P.k; g.rpA = P.rpA; g.colA = P.colA; g.rpB = P.rpB;
-            CUDA_OK(row_sample(pool, g, P.m < 4096 ? 1 : 16, rs + ST_NNZC));
-            r = host_wait(ctx, &P.nsync);
+            // where the row path is likely its products are counted at once,
+            // which saves the sample and a wait (31^3 27-point stencil 362 -> 348 us,
+            // R-MAT 2^12 x 8 A*A^T 395 -> 371); elsewhere the sample is cheaper
+            const bool ahead = P.m <= ROW_FEW && (double)P.nnzA * (double)P.nnzB <= (double)ROW_PRODUCTS * (double)P.k;
+            if (ahead) r = row_count(ctx, pool, sc, P, *rows);
+            else CUDA_OK(row_sample(pool, row_args(P), P.m < 4096 ? 1 : 16, rs + ST_NNZC, ctx->dflags));
+            if (!r) r = host_wait(ctx, &P.nsync);
             if (r) return r;
+            if (ahead) {
+                rows->counted = true;
+                memcpy(&rows->h, ctx->hstat + ST_BINS, sizeof(rows->h));
+            }
+            const long long products = ahead ? (long long)rows->h.products : ctx->hstat[ST_NNZC];
             const long long runsB = ctx->hstat[ST_TILESB], runsA = op == TSG_OP_AA ? runsB : ctx->hstat[ST_TILESA];
             order_known = true;
             unsorted = ctx->hstat[ST_BUNSORTED];
-            if (unsorted == 0 && rows_pay(P, ctx->hstat[ST_NNZC], runsA, runsB)) {
-                *by_rows = true;
+            if (unsorted == 0 && rows_pay(P, products, runsA, runsB)) {
+                rows->take = true;
                 CUDA_OK(cudaMemsetAsync(ctx->dstat, 0, sizeof(long long) * ST_HFLAGS, ctx->stream));
                 return TSG_OK;
             }
@@ -984,34 +1026,33 @@ struct RowBatch {
     int width = 0;                                  // blocks of the widest instance
 };
 
-tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double *&val, bool &taken,
+tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, int *&col, double *&val, bool &taken,
                         const RowBatch *batch = nullptr)
 {
     taken = false;
-    RowArgs g;
-    g.m = P.m; g.k = P.k; g.n = P.n; g.nblk = ceil_div_i(P.n, ROW_BLK);
-    g.rpA = P.rpA; g.rpB = P.rpB; g.colA = P.colA; g.colB = P.colB; g.valA = P.valA; g.valB = P.valB;
-    g.width = g.nblk;
-    g.sort_max = P.n <= SORT_COLS ? SORT_MAX : 0;
+    RowArgs g = row_args(P);
     if (batch) { g.base = batch->base; g.width = batch->width; g.coloff = batch->coloff; }
     Scratch sc(pool);
-    static_assert(sizeof(RowStat) <= 8 * BS_SLOTS, "the row path's statistics fit the bins' slots");
-    RowStat *rs = reinterpret_cast<RowStat *>(ctx->dstat + ST_BINS), h;
-    int *prod = sc.get<int>(P.m), *heavy = sc.get<int>((long long)HEAVY_CLASSES * P.m), *rowcnt = sc.get<int>(P.m + 1);
-    int2 *rng = sc.get<int2>(P.m);
+    RowStat *rs = reinterpret_cast<RowStat *>(ctx->dstat + ST_BINS);
+    tsg_status r = TSG_OK;
+    if (!start.counted) {
+        r = row_count(ctx, pool, sc, P, start);
+        if (!r) r = host_wait(ctx, &P.nsync);
+        if (r) return r;
+        memcpy(&start.h, ctx->hstat + ST_BINS, sizeof(start.h));
+    }
+    RowStat h = start.h;
+    const int *prod = start.prod, *heavy = start.heavy;
+    g.rng = start.rng;
+    int *rowcnt = sc.get<int>(P.m + 1);
     P.rowptrC = P.own<long long>(pool, P.m + 1);
-    if (!prod || !heavy || !rowcnt || !rng || !P.rowptrC) return fail(TSG_ERR_OOM, "device pool allocation failed (row path)");
-    g.rng = rng;
+    if (!rowcnt || !P.rowptrC) return fail(TSG_ERR_OOM, "device pool allocation failed (row path)");
     RowLanes lanes;
     lanes.fork = ctx->fork;
     for (int t = 0; t < ROW_LANES; ++t) {
         lanes.lane[t] = t == 0 ? ctx->side : ctx->lane[t - 1];
         lanes.join[t] = t == 0 ? ctx->join : ctx->lane_join[t - 1];
     }
-    CUDA_OK(row_products(pool, g, prod, rng, heavy, rs));
-    tsg_status r = host_wait(ctx, &P.nsync);
-    if (r) return r;
-    memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
     const long long cap = std::max<long long>((long long)h.items, 1);
     if ((h.seen & SEEN_BAD) || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS) return TSG_OK;
     if (h.seen & SEEN_CUTS) {   // the cut table: at most a sixteenth of the free device memory
@@ -1053,7 +1094,10 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, int *&col, double
     r = host_wait(ctx, &P.nsync);
     if (r) return r;
     P.nnzC = ctx->hstat[ST_NNZC];
-    memcpy(&h, ctx->hstat + ST_BINS, sizeof(h));
+    RowStat listed;
+    memcpy(&listed, ctx->hstat + ST_BINS, sizeof(listed));
+    std::copy(listed.front, listed.front + ITEM_CLASSES, h.front);
+    std::copy(listed.back, listed.back + ITEM_CLASSES, h.back);
     for (int c = 0; c < ITEM_CLASSES; ++c)
         if ((long long)h.front[c] + h.back[c] > cap) return fail(TSG_ERR_CUDA, "internal: the row path's items outgrew their bound");
     if (!batch && output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))
@@ -1584,12 +1628,12 @@ tsg_status tsg_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr *
     {
         Scratch sc(pool);
         // a call without statistics (of tiles and bins) may go by rows
-        bool by_rows = false;
+        RowStart rows;
         r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, st != nullptr && ctx->opts.count_products, tm, true,
-                          !st && ctx->opts.small_path ? &by_rows : nullptr);
-        if (!r && by_rows) {
+                          !st && ctx->opts.small_path ? &rows : nullptr);
+        if (!r && rows.take) {
             bool taken = false;
-            r = rows_product(ctx, pool, P, col, val, taken);
+            r = rows_product(ctx, pool, P, rows, col, val, taken);
             if (!r && taken) {
                 r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st);   // frees col and val on failure
                 P.release(pool);
@@ -2393,9 +2437,9 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         r = pack_operands(ctx, pool, sc, count, A, roff, op == TSG_OP_AAT ? koff : (op == TSG_OP_AA ? roff : koff),
                           M, op == TSG_OP_AA ? M : K, pA);
         if (!r && op == TSG_OP_AB) r = pack_operands(ctx, pool, sc, count, B, koff, noff, K, N, pB);
-        bool by_rows = false;
+        RowStart rows;
         if (!r) r = plan_symbolic(ctx, pool, sc, op, &pA, op == TSG_OP_AB ? &pB : nullptr, P, false, st != nullptr && ctx->opts.count_products, tm,
-                                  false, !st && ctx->opts.small_path ? &by_rows : nullptr);
+                                  false, !st && ctx->opts.small_path ? &rows : nullptr);
         // C's column offset of each packed tile-row's instance: the numeric
         // step writes C_i's columns already rebased
         long long rpn = 0;
@@ -2415,7 +2459,7 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         if (!r) CUDA_OK(cudaMemcpyAsync(d_trc, trc.data(), sizeof(int) * trc.size(), cudaMemcpyHostToDevice, ctx->stream));
         bool taken = false;
         std::vector<int> base;
-        if (!r && by_rows) {
+        if (!r && rows.take) {
             // per tile-row of B its instance's first block of C's columns
             RowBatch rb;
             base.assign((size_t)((op == TSG_OP_AA ? M : K) / TILE) + 1, 0);
@@ -2429,7 +2473,7 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
             if (!d_base) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch layout)");
             if (!r) CUDA_OK(cudaMemcpyAsync(d_base, base.data(), sizeof(int) * base.size(), cudaMemcpyHostToDevice, ctx->stream));
             rb.base = d_base; rb.coloff = d_trc;
-            if (!r) r = rows_product(ctx, pool, P, col, val, taken, &rb);
+            if (!r) r = rows_product(ctx, pool, P, rows, col, val, taken, &rb);
             if (!r && !taken) {
                 P.release(pool);
                 P = PlanData();

@@ -69,8 +69,9 @@ __device__ __forceinline__ bool sorted_row(const RowArgs &g, long long p, int nb
 
 // The products of every step-th row of C, times step (one warp a row).
 __global__ void __launch_bounds__(256)
-k_row_sample(RowArgs g, int step, unsigned long long *out)
+k_row_sample(RowArgs g, int step, unsigned long long *out, const int *flags)
 {
+    if (flags[FLAG_BAD_INPUT]) return;
     const long long r = (blockIdx.x * 8ll + (threadIdx.x >> 5)) * step;
     if (r >= g.m) return;
     long long p = 0;
@@ -138,8 +139,10 @@ __device__ __forceinline__ RowSum sum_entries(const RowArgs &g, const int4 *__re
 }
 
 __global__ void __launch_bounds__(256)
-k_row_products(RowArgs g, const int4 *__restrict__ ext, int *prod, int2 *rng, int *heavy, RowStat *stat)
+k_row_products(RowArgs g, const int4 *__restrict__ ext, int *prod, int2 *rng, int *heavy, RowStat *stat,
+               const int *flags)
 {
+    if (flags[FLAG_BAD_INPUT]) return;
     __shared__ unsigned long long s_p[8], s_i[8], s_b[8];
     __shared__ int s_w[8], s_lo[8], s_hi[8], s_long[WIDE_LIST], s_nlong;
     __shared__ long long s_sum[8];
@@ -1007,20 +1010,21 @@ cudaError_t rows_init_attributes()
     return e;
 }
 
-cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out)
+cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out, const int *flags)
 {
     const long long rows = (g.m + step - 1) / step;
-    k_row_sample<<<(unsigned)((rows + 7) / 8), 256, 0, pool.stream>>>(g, step, out);
+    k_row_sample<<<(unsigned)((rows + 7) / 8), 256, 0, pool.stream>>>(g, step, out, flags);
     ::tsg::count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat)
+cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat,
+                         const int *flags)
 {
     int4 *ext = pool.alloc_n<int4>(g.k);
     if (!ext) return pool.err;
     k_row_extents<<<(unsigned)((g.k + 255) / 256), 256, 0, pool.stream>>>(g.rpB, g.colB, g.k, ext);
-    k_row_products<<<warps_grid(g.m), 256, 0, pool.stream>>>(g, ext, prod, rng, heavy, stat);
+    k_row_products<<<warps_grid(g.m), 256, 0, pool.stream>>>(g, ext, prod, rng, heavy, stat, flags);
     ::tsg::count_launch();
     ::tsg::count_launch();
     pool.free(ext);

@@ -117,9 +117,10 @@ struct RowLanes {
 };
 
 cudaError_t rows_init_attributes();
+// Both may run on row pointers that the check has refused (flags), and do nothing then.
 // adds step * the products of every step-th row
-cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out);
-cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat);
+cudaError_t row_sample(Pool &pool, const RowArgs &g, int step, unsigned long long *out, const int *flags);
+cudaError_t row_products(Pool &pool, const RowArgs &g, int *prod, int2 *rng, int *heavy, RowStat *stat, const int *flags);
 cudaError_t row_cuts(Pool &pool, const RowArgs &g, int *cut);
 // items: ITEM_CLASSES lists of cap
 cudaError_t row_symbolic(Pool &pool, const RowArgs &g, const int *prod, const int *heavy, const RowStat &h,
