@@ -15,8 +15,8 @@ constexpr int KEEP_BITS = 16;               // products a block from which a row
                                               // products over 98 blocks: 2.0 ms marked again, 2.7 read back)
 constexpr int SYM_BLKS = 256;                 // blocks of the symbolic bitmap at a time (32 KB)
 constexpr int ROW_MAX_BLKS = 4096;            // blocks of a row's columns at most (4 M columns)
-constexpr int ROW_HEAVY = 1 << 15;            // rows of more products take a CTA of 1,024 threads
-constexpr int ROW_TINY = 2048;                // rows of so few products take a CTA of 64 threads
+constexpr int ROW_HEAVY = 48 << 10;           // rows of more products take a CTA of 1,024 threads
+constexpr int ROW_TINY = 4096;                // rows of so few products take a CTA of 64 threads
 constexpr int HEAVY_CLASSES = 4;              // ... listed by weight: the longest chains start first
 __host__ __device__ inline int heavy_class(long long p)
 {
