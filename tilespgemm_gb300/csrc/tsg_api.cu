@@ -45,6 +45,7 @@ cudaError_t aux_nnzcub(Pool &pool, const long long *rpA, const int *colA, int m,
 cudaError_t aux_mask_popc(Pool &pool, const int *trp, int blkm, const uint16_t *mask, unsigned long long *out);
 cudaError_t aux_rows_increasing(Pool &pool, const long long *rp, const int *col, int m, int n, long long nnz,
                                 unsigned long long *out, unsigned long long *runs);
+cudaError_t aux_run_sample(Pool &pool, const int *col, long long nnz, unsigned long long *runs);
 cudaError_t aux_copy_scalars(Pool &pool, const long long *a, long long *da, const int *b, long long *db,
                              const int *c, long long *dc);
 cudaError_t aux_rowptr_narrow(Pool &pool, const long long *in, int *out, long long n);
@@ -669,7 +670,7 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
             // tile runs of A and B, sampled products, and whether B's rows increase, decide
             unsigned long long *rs = reinterpret_cast<unsigned long long *>(ctx->dstat);
             if (op != TSG_OP_AA)
-                CUDA_OK(aux_rows_increasing(pool, P.rpA, P.colA, P.m, P.k, P.nnzA, rs + ST_NNZCUB, rs + ST_TILESA));
+                CUDA_OK(aux_run_sample(pool, P.colA, P.nnzA, rs + ST_TILESA));
             CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.n, P.nnzB, rs + ST_BUNSORTED, rs + ST_TILESB));
             // where the row path is likely its products are counted at once,
             // which saves the sample and a wait (31^3 27-point stencil 362 -> 348 us,
