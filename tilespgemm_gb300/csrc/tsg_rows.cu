@@ -27,23 +27,30 @@
 // B's rows must be strictly increasing (checked on the device by
 // k_count_descents; the tiled path takes the others).
 //
+// Short rows with wide spans are sorted instead (k_row_sort, below).
+//
 // Measured on GB300, before (tiled) and after, whole call on the device:
-//   R-MAT 2^12 x 8 A*A^T 1,190 -> 414 us, 2^15 x 16 A*A^T 8.4 -> 2.2 ms,
-//   2^16 x 12 A*A 12.9 -> 3.0 ms, 2^18 x 16 A*A^T 80 -> 35.6 ms;
-//   uniform 120,007 x 80,021 x 100,003, 16 and 12 a row: 10.3 -> 2.0 ms;
-//   512 mixed products of 64 to 16,384 rows: 41.7 -> 24.5 ms.
-// What bounds it (2^15, counters): k_row_numeric, 2/3 of the time, by issue
-// and by the latency of a step's chain (B's entry, its word, its accumulator,
-// the fma): 28 instructions a step and 7 to stage it, 1.1 to 1.6 a clock and
-// SM, FP64 pipe 20-30 % busy; marking an item's columns again cost another 28
-// a step (2^18: 41.0 ms without kept bitmaps).  k_row_symbolic is bound by its
-// bitmap's shared-memory accesses.
-// Tried without gain: products flattened 32 at a time over an item's shares,
-// lanes that meet ordered by rank (2^18: 77 ms; R-MAT's columns meet in
-// nearly every round); items of 6,144 entries as a CTA's, 128 entries a step
-// (67 ms: idle warps and a barrier a step); groups of 2 or 8 steps in flight
-// in place of 4 (50 / 58 against 45 ms: loads exposed, code outgrows the
-// instruction cache).
+//   R-MAT 2^12 x 8 A*A^T 1,170 -> 373 us, 2^15 x 16 A*A^T 8.9 -> 1.5 ms,
+//   2^16 x 12 A*A 12.9 -> 2.45 ms, 2^18 x 16 A*A^T 81 -> 35 ms;
+//   uniform 120,007 x 80,021 x 100,003, 16 and 12 a row: 10.3 -> 0.59 ms;
+//   512 mixed products of 64 to 16,384 rows: 41.9 -> 23.3 ms.
+// What bounds it (2^16, counters): k_row_numeric, 2/3 of the time: FP64 pipe 46
+// to 56 % busy (a step holds it as long with 3 lanes as with 32; 2^18: half of
+// the 211 M steps bring 8 entries or fewer), issue 39 to 44 %, and between
+// them the latency of a step's chain (B's entry, its word, its accumulator,
+// the fma) over the 14 to 20 warps that an SM's shared memory holds: 28
+// instructions a step and 7 to stage it; marking an item's columns again cost
+// another 28 (2^18: 41.0 ms without kept bitmaps).  k_row_symbolic is bound by
+// its bitmap's shared-memory accesses and, for short rows, by a row's fixed cost.
+// Tried without gain: products flattened 32 at a time over an item's A
+// entries, half the rounds, lanes that meet in a column ordered by match (2^18:
+// 77 ms; a match costs 2 clocks a distinct value and SM), by atomicMin in a
+// table of 512 slots (37.3 for 34.8 ms: its 2 KB cost two warps an SM), or one
+// A entry after another (34.5 to 37.7; 512 mixed products 28 for 24.4); items
+// of 6,144 entries as a CTA's, 128 entries a step (67 ms: idle warps and a
+// barrier a step); groups of 2 or 8 steps in flight in place of 4 (50 / 58
+// against 45 ms: loads exposed, code outgrows the instruction cache); 24
+// warps an SM at 80 registers, or a finer list of classes (within 2 %).
 // The reference bins C's rows by intermediate products for its tile-level
 // symbolic step (spgemm_nsparse_kernel.h:32-311); it has no row path.
 #include "tsg_internal.cuh"

@@ -19,6 +19,11 @@
 //                  kept count, or that is over the limit, adds 1 to kept[0]
 //                  (the caller then runs the count pass), the products go
 //                  to kept[1].
+//   k_small_fill_one  the same for a repeated shape whose rows of A have up to
+//                  32 entries and bring up to 32 products: a warp takes four
+//                  rows (one where there are few), whose loads share their
+//                  latencies, and the last CTA writes the counts and flags to
+//                  the host's memory, so that the call is one launch and one wait
 // The row's products are dealt 32 at a time in A's order then B's (lane =
 // position in the concatenation of the B rows of up to 32 A entries); lanes
 // of one round that meet in one output apply in lane order, so every entry
