@@ -89,6 +89,14 @@ def test_rows_match_oracle_and_tiles(rctx, ctx, name):
     _check(ctx.spgemm(A, B, op=op), ref)       # the tiled pipeline
 
 
+def test_rows_many_products_match_tiles(rctx, ctx):
+    """Over 400 M products: rows of up to 2,048 entries are light, not 4,096."""
+    A = _rows(13000, 8000, [6, 7, 12, 15, 16, 230, 230, 230], 30)
+    B = _rows(8000, 8200, [360], 31)
+    C, D = rctx.spgemm(A, B, op="AB"), ctx.spgemm(A, B, op="AB")
+    _check(C, (np.asarray(D.rowptr, np.int64), D.col, D.val))
+
+
 @pytest.mark.parametrize("bits", [32, 64])
 def test_rows_device_operands_and_output(rctx, bits):
     import torch

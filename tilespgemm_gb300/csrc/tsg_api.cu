@@ -1056,7 +1056,9 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, 
     }
     const long long cap = std::max<long long>((long long)h.items, 1);
     if ((h.seen & SEEN_BAD) || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS) return TSG_OK;
-    if (h.seen & SEEN_CUTS) {   // the cut table: at most a sixteenth of the free device memory
+    const bool many = (long long)h.products > MANY_PRODUCTS;
+    if (many) g.light = LIGHT_MANY;
+    if (h.seen & (many ? SEEN_CUTS | SEEN_MANY : SEEN_CUTS)) {   // the cut table: at most a sixteenth of the free device memory
         const long long n = (long long)P.k * (g.width + 1);
         size_t free_b = 0, total_b = 0;
         if (4 * n > (64ll << 20) &&

@@ -31,9 +31,9 @@
 //
 // Measured on GB300, before (tiled) and after, whole call on the device:
 //   R-MAT 2^12 x 8 A*A^T 1,170 -> 373 us, 2^15 x 16 A*A^T 8.9 -> 1.5 ms,
-//   2^16 x 12 A*A 12.9 -> 2.45 ms, 2^18 x 16 A*A^T 81 -> 35 ms;
+//   2^16 x 12 A*A 12.9 -> 2.45 ms, 2^18 x 16 A*A^T 81 -> 33.5 ms;
 //   uniform 120,007 x 80,021 x 100,003, 16 and 12 a row: 10.3 -> 0.59 ms;
-//   512 mixed products of 64 to 16,384 rows: 41.9 -> 23.3 ms.
+//   512 mixed products of 64 to 16,384 rows: 41.9 -> 22.6 ms.
 // What bounds it (2^16, counters): k_row_numeric, 2/3 of the time: FP64 pipe 46
 // to 56 % busy (a step holds it as long with 3 lanes as with 32; 2^18: half of
 // the 211 M steps bring 8 entries or fewer), issue 39 to 44 %, and between
@@ -173,6 +173,7 @@ k_row_products(RowArgs g, const int4 *__restrict__ ext, int *prod, int2 *rng, in
             if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
             si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
             if (p > LIGHT_ROW || nb > SYM_BLKS) seen |= SEEN_CUTS;
+            if (p > LIGHT_MANY) seen |= SEEN_MANY;
         }
         if (s.out) seen |= SEEN_BAD;
         if (p > ROW_HEAVY) {
@@ -440,10 +441,10 @@ k_row_symbolic(RowArgs g, const int *__restrict__ prod, int p0, int p1, HeavyRow
         for (int j = lane; j < nblk; j += 32) t += cnt[j];
         t = warp_sum_int(t);
         if (lane == 0) { cnt[nblk] = t; rowcnt[r] = t; }
-        if (t <= LIGHT_ROW) { tclose = LIGHT_ROW + 1; bmax = LIGHT_BLKS; }
+        if (t <= g.light) { tclose = LIGHT_ROW + 1; bmax = LIGHT_BLKS; }
         __syncwarp();
     }
-    if (cnt[nblk] <= LIGHT_ROW && nblk <= LIGHT_BLKS) {      // one item
+    if (cnt[nblk] <= g.light && nblk <= LIGHT_BLKS) {      // one item
         const int z = cnt[nblk];
         if (lane == 0 && z > 0) {
             const int c = item_class(z, nblk, (float)p <= g.each * (float)la);

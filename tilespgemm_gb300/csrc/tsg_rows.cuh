@@ -9,6 +9,13 @@ constexpr int ITEM_T = 1024;                  // an item closes once its row's e
 constexpr int ITEM_CAP = ITEM_T + ROW_BLK;    // entries of an item at most (a block adds at most ROW_BLK)
 constexpr int ITEM_BLKS = 16;                 // blocks of an item at most
 constexpr int LIGHT_ROW = 4096, LIGHT_BLKS = 256;   // rows of so few entries: one item per so many blocks
+// ... of a product of more than MANY_PRODUCTS, which fills the GPU without the
+// light rows' CTAs of 128 threads (R-MAT 2^18 x 16 A*A^T 34.3 ms a call with
+// 4,096, 33.5 with 2,048; 512 mixed products, 2.1 G: 23.1 and 22.5, 23.4 with
+// 1,024); below it those shorten the longest chains (R-MAT 2^12 x 8 379 us with
+// 4,096, 392 with 2,048; 2^15 x 16 1,498 and 1,533)
+constexpr int LIGHT_MANY = 2048;
+constexpr long long MANY_PRODUCTS = 400000000;
 constexpr int KEEP_BITS = 16;               // products a block from which a row's bitmap is kept for the numeric
                                               // pass (and entries a block from which an item reads it: 128 bytes a
                                               // block against 8 an entry; with none of its own, uniform rows of 192
@@ -72,6 +79,7 @@ struct RowArgs {
     const long long *rpA = nullptr, *rpB = nullptr;
     const int *colA = nullptr, *colB = nullptr;
     const double *valA = nullptr, *valB = nullptr;
+    int light = LIGHT_ROW;                    // rows of so many entries at most are light
     int sort_max = 0;                         // rows of so many products at most are sorted (0: none)
     float each = 32;                          // light rows: products of an A entry from which an item is a CTA's
     const int2 *rng = nullptr;                // each row of C: its blocks [x, y)
@@ -94,6 +102,7 @@ struct RowArgs {
 // What row_products finds (zeroed before).
 constexpr unsigned SEEN_BAD = 1;     // a column of A outside B's rows
 constexpr unsigned SEEN_CUTS = 2;    // a row needs the cut table (more than one item or window)
+constexpr unsigned SEEN_MANY = 32;   // the same were LIGHT_MANY the line
 constexpr unsigned SEEN_SORT = 4;    // rows of up to 128 (<< 1: 256, << 2: SORT_MAX) products to sort
 
 struct RowStat {
