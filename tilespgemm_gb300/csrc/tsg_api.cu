@@ -674,17 +674,22 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
             CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.n, P.nnzB, rs + ST_BUNSORTED, rs + ST_TILESB));
             // where the row path is likely its products are counted at once,
             // which saves the sample and a wait (31^3 27-point stencil 362 -> 348 us,
-            // R-MAT 2^12 x 8 A*A^T 395 -> 371); elsewhere the sample is cheaper
-            const bool ahead = P.m <= ROW_FEW && (double)P.nnzA * (double)P.nnzB <= (double)ROW_PRODUCTS * (double)P.k;
+            // R-MAT 2^12 x 8 A*A^T 395 -> 371); elsewhere the sample is cheaper,
+            // and needless where the averages, which skew only adds to, put the
+            // products past both lines (96^3 27-point stencil 3,830 -> 3,774 us)
+            const double mean = (double)P.nnzA * (double)P.nnzB / (double)P.k;
+            const bool ahead = P.m <= ROW_FEW && mean <= (double)ROW_PRODUCTS;
+            const bool plain = mean > (double)ROW_PRODUCTS && mean >= 128.0 * P.m;
             if (ahead) r = row_count(ctx, pool, sc, P, *rows);
-            else CUDA_OK(row_sample(pool, row_args(P), P.m < 4096 ? 1 : 16, rs + ST_NNZC, ctx->dflags));
+            else if (!plain) CUDA_OK(row_sample(pool, row_args(P), P.m < 4096 ? 1 : 16, rs + ST_NNZC, ctx->dflags));
             if (!r) r = host_wait(ctx, &P.nsync);
             if (r) return r;
             if (ahead) {
                 rows->counted = true;
                 memcpy(&rows->h, ctx->hstat + ST_BINS, sizeof(rows->h));
             }
-            const long long products = ahead ? (long long)rows->h.products : ctx->hstat[ST_NNZC];
+            const long long products = ahead ? (long long)rows->h.products
+                                     : plain ? (long long)std::min(mean, 9e18) : ctx->hstat[ST_NNZC];
             const long long runsB = ctx->hstat[ST_TILESB], runsA = op == TSG_OP_AA ? runsB : ctx->hstat[ST_TILESA];
             order_known = true;
             unsorted = ctx->hstat[ST_BUNSORTED];
