@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -666,7 +667,9 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
     long long unsorted = 0;
     if (rows) {
         *rows = RowStart();
-        if (P.nnzA > 0 && P.nnzB > 0) {
+        // the row path's 32-bit positions step past a row's end by less than this
+        const long long most = INT_MAX - (1 << 16);
+        if (P.nnzA > 0 && P.nnzB > 0 && std::max({(long long)P.m, (long long)P.k, (long long)P.n, P.nnzA, P.nnzB}) <= most) {
             // tile runs of A and B, sampled products, and whether B's rows increase, decide
             unsigned long long *rs = reinterpret_cast<unsigned long long *>(ctx->dstat);
             if (op != TSG_OP_AA)
