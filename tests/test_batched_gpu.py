@@ -8,6 +8,15 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(scope="module")
+def rows_ctx(built_lib):
+    """A context with its defaults: batches may go by rows."""
+    from tilespgemm_gb300 import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
 def _instances(count, seed, square=True):
     from tilespgemm_gb300 import matrices as M
     rng = np.random.default_rng(seed)
@@ -109,3 +118,40 @@ def test_sibling_results_freed_from_many_threads(ctx):
     finally:
         for oc in first + second:
             oc.free()
+
+
+@pytest.mark.parametrize("op", ["AA", "AAT", "AB"])
+@pytest.mark.parametrize("strided", [(0,), (1,), (5,), (0, 1, 5)])
+def test_batched_strided_device_operands(rows_ctx, op, strided):
+    """Instances whose arrays torch has to copy first (every second element of
+    a longer tensor, filled behind work queued on torch's stream): the product
+    starts behind the copies of all instances."""
+    import torch
+    from tilespgemm_gb300 import matrices as M
+    from tilespgemm_gb300.api import CSR
+
+    def device(X, i):
+        if i not in strided:
+            return X.to_device(0)
+        out = []
+        for a in (X.rowptr, X.col, X.val):
+            a = np.asarray(a)
+            t = torch.zeros(2 * a.size, dtype=getattr(torch, str(a.dtype)), device="cuda")
+            t[::2] = torch.as_tensor(a).to("cuda")
+            out.append(t[::2])
+        return CSR(X.m, X.n, *out)
+
+    As = [M.random_sparse(200 + 30 * i, 200 + 30 * i + (0 if op == "AA" else 7), 6, seed=70 + i) for i in range(6)]
+    Bs = [M.random_sparse(A.n, 150 + 40 * i, 5, seed=90 + i) for i, A in enumerate(As)] if op == "AB" else None
+    big = torch.ones(1 << 27, device="cuda")
+    for _ in range(8):
+        big.mul_(1.0)
+    dA = [device(A, i) for i, A in enumerate(As)]
+    dB = [device(B, i) for i, B in enumerate(Bs)] if Bs else None
+    outs, _ = rows_ctx.spgemm_batched_raw(dA, dB, op=op, out="device")
+    for i, (A, oc) in enumerate(zip(As, outs)):
+        B = Bs[i] if Bs else A
+        if op == "AAT":
+            B = CSR(A.n, A.m, *O.transpose(A))
+        _check(oc.download(), A, B)
+        oc.free()

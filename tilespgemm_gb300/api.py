@@ -65,11 +65,12 @@ class CSR:
         return CSR(self.m, self.n, torch.as_tensor(np.asarray(self.rowptr)).to(dev),
                    torch.as_tensor(np.asarray(self.col)).to(dev), torch.as_tensor(np.asarray(self.val)).to(dev))
 
-    def _tsg(self, ctx_handle=None, synced: bool = False) -> tuple[_abi.tsg_csr, list]:
+    def _tsg(self, ctx_handle=None, wait: bool = True) -> tuple[_abi.tsg_csr, list]:
         """tsg_csr view of this matrix plus the objects that must stay alive.
         Device tensors: the context's stream (ctx_handle) is ordered after
         torch's current stream without blocking; without a context the host
-        waits for torch's stream (synced: it has already)."""
+        waits for torch's stream, which copies strided tensors here (wait
+        False: the caller does, behind the last of its views)."""
         s = _abi.tsg_csr()
         s.m, s.n = int(self.m), int(self.n)
         keep: list = []
@@ -87,7 +88,7 @@ class CSR:
             s.nnz = col.numel()
             if ctx_handle:
                 check(lib().tsg_stream_wait(ctx_handle, torch.cuda.current_stream(rp.device).cuda_stream))
-            elif not synced:
+            elif wait:
                 torch.cuda.current_stream(rp.device).synchronize()
         else:
             rp = np.asarray(self.rowptr)
@@ -105,6 +106,28 @@ class CSR:
             s.nnz = int(col.size)
         s.owner = None
         return s, keep
+
+
+def _tsg_list(Xs: list, n: int) -> tuple[Any, list, set]:
+    """tsg_csr views of Xs in one array of n, the objects that must stay
+    alive, and the devices whose torch streams the caller has to wait for."""
+    arr = (_abi.tsg_csr * max(n, 1))()
+    keep: list = []
+    devices = set()
+    for i, X in enumerate(Xs):
+        arr[i], k = X._tsg(wait=False)
+        keep.append(k)
+        if X.on_device:
+            devices.add(k[0].device)
+    return arr, keep, devices
+
+
+def _wait_torch(devices: set) -> None:
+    """The host waits for torch's current stream on each of these devices."""
+    if devices:
+        import torch
+        for d in devices:
+            torch.cuda.current_stream(d).synchronize()
 
 
 def _download(ctx_handle, s: _abi.tsg_csr) -> CSR:
@@ -409,25 +432,17 @@ class Context:
         """C_i = op(A_i, B_i) for all instances in one pipeline pass (tsg_spgemm_batched);
         returns OwnedCSR views that share one allocation."""
         n = len(As)
-        a = (_abi.tsg_csr * max(n, 1))()
-        keep: list = []
-        for i, A in enumerate(As):
-            s_, k_ = A._tsg(synced=i > 0)
-            a[i] = s_
-            keep.append(k_)
-        b_ptr = None
+        a, keep_a, devices = _tsg_list(As, n)
+        b_ptr, keep_b = None, None
         if Bs is not None:
-            b = (_abi.tsg_csr * max(n, 1))()
-            for i, B in enumerate(Bs):
-                s_, k_ = B._tsg(synced=n > 0)
-                b[i] = s_
-                keep.append(k_)
-            b_ptr = b
+            b_ptr, keep_b, more = _tsg_list(Bs, n)
+            devices |= more
+        _wait_torch(devices)      # once, behind the copies of every strided tensor
         c = (_abi.tsg_csr * max(n, 1))()
         c[0].where = _abi.MEM_DEVICE if out == "device" else _abi.MEM_HOST
         st = _abi.tsg_stats() if stats else None
         check(lib().tsg_spgemm_batched(self.handle, _OPS[op], n, a, b_ptr, c, C.byref(st) if st is not None else None))
-        del keep
+        del keep_a, keep_b
         outs = [OwnedCSR(self, c[i]) for i in range(n)]
         return outs, (st.as_dict() if st is not None else None)
 
