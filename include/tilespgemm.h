@@ -150,6 +150,11 @@ const char *tsg_version(void);
  * around the library's kernels.  tsg_measure_fp64_peak: the device's FP64
  * FMA throughput in GFLOP/s (2 FLOP per FMA), measured by a short kernel. */
 int64_t tsg_launch_count(void);
+
+/* Products (tsg_spgemm calls, and batches as one) that ran row by row in this
+ * process instead of through the tiles: the two give the same bits, so only
+ * this tells them apart (no counterpart in the reference). */
+int64_t tsg_row_path_count(void);
 void *tsg_get_stream(tsg_ctx *ctx);
 
 /* Order the context's stream after the work already queued on `stream` (a

@@ -104,6 +104,7 @@ SIGNATURES = {
     "tsg_last_error": (C.c_char_p, []),
     "tsg_version": (C.c_char_p, []),
     "tsg_launch_count": (C.c_int64, []),
+    "tsg_row_path_count": (C.c_int64, []),
     "tsg_pinned_cache_cap": (C.c_int64, []),
     "tsg_get_stream": (C.c_void_p, [C.c_void_p]),
     "tsg_stream_wait": (C.c_int, [C.c_void_p, C.c_void_p]),

@@ -93,6 +93,7 @@ using namespace tsg;
 
 static thread_local std::string g_err;
 static std::atomic<long long> g_launches{0};
+static std::atomic<long long> g_row_products{0};   // tsg_row_path_count
 
 void tsg::count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
@@ -1118,6 +1119,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, 
     if (!col || !val) return fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
     P.wait_values(ctx->stream);
     CUDA_OK(row_numeric(pool, g, prod, items, (unsigned)cap, h, P.rowptrC, col, val, ctx->dflags, lanes));
+    g_row_products.fetch_add(1, std::memory_order_relaxed);
     taken = true;
     return TSG_OK;
 }
@@ -1437,6 +1439,8 @@ const char *tsg_last_error(void) { return g_err.c_str(); }
 const char *tsg_version(void) { return "tilespgemm-gb300 0.1 (sm_103a)"; }
 
 int64_t tsg_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+
+int64_t tsg_row_path_count(void) { return g_row_products.load(std::memory_order_relaxed); }
 
 int64_t tsg_pinned_cache_cap(void) { return (int64_t)pinned_cap(); }
 
