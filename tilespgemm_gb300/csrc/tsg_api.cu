@@ -108,6 +108,16 @@ bool tsg::alloc_should_fail(int kind)
     return c.fetch_sub(1, std::memory_order_relaxed) == 1;
 }
 
+// the numeric steps still to go before the one that reports a failed check
+// (tsg_inject_check_failure); 0 or below: disarmed
+static std::atomic<long long> g_fail_check{0};
+
+static bool check_should_fail()
+{
+    if (g_fail_check.load(std::memory_order_relaxed) <= 0) return false;
+    return g_fail_check.fetch_sub(1, std::memory_order_relaxed) == 1;
+}
+
 namespace tsg {
 void set_last_error(const char *msg) { g_err = msg; }
 void noalloc_forget(int device);
@@ -429,6 +439,21 @@ tsg_status read_flags(tsg_ctx *ctx)
     return TSG_OK;
 }
 
+// device -> pinned mirror of the flags alone, read by flags_arrived after a wait
+cudaError_t flags_down(tsg_ctx *ctx)
+{
+    return cudaMemcpyAsync(ctx->hstat + ST_HFLAGS, ctx->dflags, sizeof(int) * FLAG_COUNT, cudaMemcpyDeviceToHost,
+                           ctx->stream);
+}
+
+tsg_status flags_arrived(tsg_ctx *ctx)
+{
+    int hflags[FLAG_COUNT];
+    memcpy(hflags, ctx->hstat + ST_HFLAGS, sizeof(hflags));
+    for (int f = 0; f < FLAG_COUNT; ++f) ctx->hstat[ST_HFLAGS + f] = hflags[f];
+    return read_flags(ctx);
+}
+
 // device -> pinned mirror of stats and flags, then wait
 tsg_status host_wait(tsg_ctx *ctx, int *nsync)
 {
@@ -439,12 +464,9 @@ tsg_status host_wait(tsg_ctx *ctx, int *nsync)
     static_assert(sizeof(SmallReport) <= 8 * (ST_SLOTS - ST_REPORT) && 2 + FLAG_COUNT <= ST_SLOTS - ST_REPORT, "report");
     static_assert(ST_BINS + BS_SLOTS <= ST_BUNSORTED && ST_BUNSORTED < ST_SMALL && ST_SMALL + 3 <= ST_HFLAGS,
                   "statistics slots");
-    int hflags[FLAG_COUNT];
     CUDA_OK(cudaStreamSynchronize(ctx->stream));
-    memcpy(hflags, ctx->hstat + ST_HFLAGS, sizeof(hflags));
-    for (int f = 0; f < FLAG_COUNT; ++f) ctx->hstat[ST_HFLAGS + f] = hflags[f];
     if (nsync) ++*nsync;
-    return read_flags(ctx);
+    return flags_arrived(ctx);
 }
 
 double ms_since(std::chrono::steady_clock::time_point t0)
@@ -840,6 +862,7 @@ tsg_status plan_numeric(tsg_ctx *ctx, Pool &pool, PlanData &P, const double *val
     else if (walk == 0 && P.nnzC > 0 && P.k > 0 &&
              (double)P.nnzA * ((double)P.nnzB / P.k) < 3.0 * (double)P.nnzC) kw = 2;
     CUDA_OK(numeric_run(pool, na, P.bstat, kw, threads, ctx->opts.row_warps, ctx->side, ctx->fork, ctx->join));
+    if (check_should_fail()) CUDA_OK(cudaMemsetAsync(ctx->dflags + FLAG_INTERNAL, 1, sizeof(int), ctx->stream));
     return TSG_OK;
 }
 
@@ -938,9 +961,12 @@ void early_out_abort(tsg_ctx *ctx, Pool &pool, EarlyOut &eo)
 
 // Hand C (rowptr copied/narrowed from `rowptr`, col/val adopted) to the
 // caller per C->where; frees col/val on failure.  With `eo` (host output
-// begun by early_out_begin) only the values remain to be copied.
+// begun by early_out_begin) only the values remain to be copied.  The flags
+// that the numeric kernels set come along with the wait: a row that did not
+// fit the symbolic pass's count is an error and no result (`checked`: the
+// caller has read them).
 tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, const long long *rowptr, int *col,
-                       double *val, tsg_csr *C, tsg_stats *st, EarlyOut *eo = nullptr)
+                       double *val, tsg_csr *C, tsg_stats *st, EarlyOut *eo = nullptr, bool checked = false)
 {
     if (eo && eo->on) {
         auto t_d2h = std::chrono::steady_clock::now();
@@ -951,6 +977,7 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
         cudaError_t e = cudaMemcpyAsync(eo->hval, val, eo->vb, cudaMemcpyDeviceToHost, ctx->stream);
         cudaStreamWaitEvent(ctx->stream, ctx->copy_done, 0);
         pool.free(eo->rp_dev); pool.free(col); pool.free(val);
+        if (e == cudaSuccess && !checked) e = flags_down(ctx);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         o->blocks.push_back({eo->hrp, eo->rpb});
         o->blocks.push_back({eo->hcol, eo->cb});
@@ -965,7 +992,9 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
             cudaGetLastError();
             return fail(cuda_status(e), "output: %s", cudaGetErrorString(e));
         }
-        return TSG_OK;
+        const tsg_status r = checked ? TSG_OK : flags_arrived(ctx);
+        if (r) tsg_csr_free(ctx, C);
+        return r;
     }
     const int bits = output_bits(ctx, nnzC);
     if (bits == 32 && nnzC >= (1ll << 31)) {
@@ -984,6 +1013,7 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
         o->blocks.push_back({col, 0});
         o->blocks.push_back({val, 0});
         C->row_ptr = rp_dev; C->col = col; C->val = val;
+        if (e == cudaSuccess && !checked) e = flags_down(ctx);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     } else {
         auto t_d2h = std::chrono::steady_clock::now();
@@ -995,6 +1025,7 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
         if (e == cudaSuccess && nnzC > 0) e = cudaMemcpyAsync(hcol, col, cb, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess && nnzC > 0) e = cudaMemcpyAsync(hval, val, vb, cudaMemcpyDeviceToHost, ctx->stream);
         pool.free(rp_dev); pool.free(col); pool.free(val);
+        if (e == cudaSuccess && !checked) e = flags_down(ctx);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (hrp) o->blocks.push_back({hrp, rpb});
         if (hcol) o->blocks.push_back({hcol, cb});
@@ -1009,7 +1040,9 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
         cudaGetLastError();
         return fail(e == cudaErrorMemoryAllocation ? TSG_ERR_OOM : TSG_ERR_CUDA, "output: %s", cudaGetErrorString(e));
     }
-    return TSG_OK;
+    const tsg_status r = checked ? TSG_OK : flags_arrived(ctx);
+    if (r) tsg_csr_free(ctx, C);
+    return r;
 }
 
 void phase_times(tsg_ctx *ctx, tsg_stats *st, const PhaseTimer &tm)
@@ -1119,6 +1152,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, 
     if (!col || !val) return fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
     P.wait_values(ctx->stream);
     CUDA_OK(row_numeric(pool, g, prod, items, (unsigned)cap, h, P.rowptrC, col, val, ctx->dflags, lanes));
+    if (check_should_fail()) CUDA_OK(cudaMemsetAsync(ctx->dflags + FLAG_INTERNAL, 1, sizeof(int), ctx->stream));
     g_row_products.fetch_add(1, std::memory_order_relaxed);
     taken = true;
     return TSG_OK;
@@ -1389,7 +1423,7 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
         C->owner = o;
         P.release(pool);
     } else {
-        r = emit_output(ctx, pool, P.m, P.n, nnzC, rowptr, col, val, C, st);   // frees col and val
+        r = emit_output(ctx, pool, P.m, P.n, nnzC, rowptr, col, val, C, st, nullptr, true);   // frees col and val
         P.release(pool);
         if (r) { cudaStreamSynchronize(ctx->stream); return r; }
         if (st) st->n_syncs = 1;
@@ -1460,6 +1494,13 @@ tsg_status tsg_inject_alloc_failure(int32_t kind, int64_t countdown)
     if (kind != 0 && kind != 1) return fail(TSG_ERR_INVALID_ARG, "kind must be 0 (device pool) or 1 (pinned host)");
     if (countdown < 0) return fail(TSG_ERR_INVALID_ARG, "countdown must be >= 0");
     g_fail_alloc[kind].store(countdown, std::memory_order_relaxed);
+    return TSG_OK;
+}
+
+tsg_status tsg_inject_check_failure(int64_t countdown)
+{
+    if (countdown < 0) return fail(TSG_ERR_INVALID_ARG, "countdown must be >= 0");
+    g_fail_check.store(countdown, std::memory_order_relaxed);
     return TSG_OK;
 }
 
@@ -1805,10 +1846,6 @@ tsg_status tsg_plan_execute(tsg_ctx *ctx, tsg_plan *plan, const double *valA, co
     fill_stats(P, st);
     r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st, &eo);
     if (r) return r;
-    // numeric kernels report an internal bound failure through the flags
-    int hflags[FLAG_COUNT];
-    CUDA_OK(cudaMemcpy(hflags, ctx->dflags, sizeof(hflags), cudaMemcpyDeviceToHost));
-    if (hflags[FLAG_INTERNAL]) { tsg_csr_free(ctx, C); return fail(TSG_ERR_CUDA, "internal bound check failed on the device"); }
     if (st) { st->ms_total = ms_since(t0); st->n_syncs = 1; }
     return TSG_OK;
 }
