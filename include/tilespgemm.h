@@ -188,6 +188,10 @@ tsg_status tsg_measure_fp64_peak(tsg_ctx *ctx, double *gflops);
  *   what its kernels report when an entry of C does not fit the symbolic
  *   pass's structure (the flag is set behind them); the call returns
  *   TSG_ERR_CUDA and no result.  Process-wide; countdown 0 disarms it.
+ * tsg_inject_free_memory: the row path sees so many bytes of free device
+ *   memory when it decides whether its tables fit (without room for the kept
+ *   bitmaps it makes them again, without room for the others the product goes
+ *   through the tiles).  Process-wide; a negative count disarms it.
  * tsg_check_bounded_wait: runs the library's single-pass device scan over n
  *   ones with its look-back waits limited to spin_limit polls, set up so
  *   that the first tile's sum is never published (no CTA takes tile 0).  The waits for it give up, the kernel finishes, and the
@@ -197,6 +201,7 @@ tsg_status tsg_measure_fp64_peak(tsg_ctx *ctx, double *gflops);
 tsg_status tsg_inject_alloc_failure(int32_t kind, int64_t countdown);
 int64_t tsg_alloc_failure_pending(int32_t kind);
 tsg_status tsg_inject_check_failure(int64_t countdown);
+tsg_status tsg_inject_free_memory(int64_t bytes);
 tsg_status tsg_check_bounded_wait(tsg_ctx *ctx, int64_t n, int32_t spin_limit);
 
 /* ---- matrix market load path ------------------------------------------- */

@@ -104,3 +104,36 @@ def test_batches_by_rows_on_the_device(rctx, op):  # noqa: F811
     for i, (A, oc) in enumerate(zip(As, outs)):
         _check(oc.download(), O.spgemm(A, _b(A, Bs[i] if Bs else None, op)))
         oc.free()
+
+
+@pytest.fixture()
+def free_memory():
+    from tilespgemm_gb300 import _abi
+    L = _abi.lib()
+    yield lambda n: _abi.check(L.tsg_inject_free_memory(n))
+    L.tsg_inject_free_memory(-1)
+
+
+@pytest.mark.parametrize("name", ["one_block", "many_blocks", "heavy_windows", "rmat9", "sort_classes"])
+def test_tables_without_room(rctx, free_memory, name):  # noqa: F811
+    """With more and more free memory: first by tiles, then by rows with the
+    bitmaps made again, then with them kept; always the same C."""
+    A, B, op = _cases()[name]
+    ref = O.spgemm(A, _b(A, B, op))
+    ways = []
+    for n in [0] + [1 << e for e in range(10, 44, 3)]:
+        free_memory(n)
+        C, went = _went(lambda: rctx.spgemm(A, B, op=op))
+        _check(C, ref)
+        ways.append(went)
+    assert ways[0] == 0 and ways[-1] == 1 and ways == sorted(ways)
+
+
+def test_items_of_light_rows_fit_their_bound(rctx):  # noqa: F811
+    """Rows of few entries over more than 256 and 512 blocks: two and three
+    items each, as many as their bound; also with rows past LIGHT_MANY among them."""
+    for n in (300007, 600011):
+        A, B = _rows(700, 400, [25, 30, 26, 90], 85), _rows(400, n, [22, 31, 25], 86)
+        C, went = _went(lambda: rctx.spgemm(A, B, op="AB"))
+        assert went == 1
+        _check(C, O.spgemm(A, B))

@@ -118,6 +118,21 @@ static bool check_should_fail()
     return g_fail_check.fetch_sub(1, std::memory_order_relaxed) == 1;
 }
 
+// the free device memory that the row path's tables see (tsg_inject_free_memory); below 0: the device's
+static std::atomic<long long> g_free_memory{-1};
+
+// Whether a table of the row path may take so many bytes: at most a sixteenth
+// of the free device memory, which a small one need not ask for.
+static bool table_fits(long long bytes)
+{
+    const long long told = g_free_memory.load(std::memory_order_relaxed);
+    if (told >= 0) return bytes <= told / 16;
+    if (bytes <= (64ll << 20)) return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return false; }
+    return bytes <= (long long)(free_b / 16);
+}
+
 namespace tsg {
 void set_last_error(const char *msg) { g_err = msg; }
 void noalloc_forget(int device);
@@ -1097,17 +1112,13 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, 
         lanes.join[t] = t == 0 ? ctx->join : ctx->lane_join[t - 1];
     }
     const long long cap = std::max<long long>((long long)h.items, 1);
-    if ((h.seen & SEEN_BAD) || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS) return TSG_OK;
+    const long long item_bytes = 16ll * ITEM_CLASSES * cap;
+    if ((h.seen & SEEN_BAD) || cap >= (1ll << 30) || h.width > ROW_MAX_BLKS || !table_fits(item_bytes)) return TSG_OK;
     const bool many = (long long)h.products > MANY_PRODUCTS;
     if (many) g.light = LIGHT_MANY;
-    if (h.seen & (many ? SEEN_CUTS | SEEN_MANY : SEEN_CUTS)) {   // the cut table: at most a sixteenth of the free device memory
+    if (h.seen & (many ? SEEN_CUTS | SEEN_MANY : SEEN_CUTS)) {   // the cut table
         const long long n = (long long)P.k * (g.width + 1);
-        size_t free_b = 0, total_b = 0;
-        if (4 * n > (64ll << 20) &&
-            (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 4 * n > (long long)(free_b / 16))) {
-            cudaGetLastError();
-            return TSG_OK;
-        }
+        if (!table_fits(4 * n)) return TSG_OK;
         int *cut = sc.get<int>(n);
         if (!cut) return fail(TSG_ERR_OOM, "device pool allocation failed (cut table)");
         CUDA_OK(row_cuts(pool, g, cut));
@@ -1120,17 +1131,10 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, 
     // SMs are full (512 mixed products: 30.7 ms with 64, 36.6 with 32, 39.1 with 200)
     g.each = h.products > 24000000 ? 64.0f : 32.0f;
     if (!items) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's items)");
-    {   // the rows' bitmaps kept for the numeric pass: at most a sixteenth of the free device memory
-        const long long bytes = 128ll * (long long)h.blocks;
-        size_t free_b = 0, total_b = 0;
-        if (h.blocks < (1ull << 31) &&
-            (bytes <= (64ll << 20) ||
-             (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && bytes <= (long long)(free_b / 16)))) {
-            g.bits = sc.get<unsigned>(32ll * (long long)h.blocks);
-            g.bitoff = sc.get<int>(P.m);
-            if (!g.bits || !g.bitoff) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's bitmaps)");
-        }
-        cudaGetLastError();
+    if (h.blocks < (1ull << 31) && table_fits(128ll * (long long)h.blocks)) {   // the rows' bitmaps, kept for the numeric pass
+        g.bits = sc.get<unsigned>(32ll * (long long)h.blocks);
+        g.bitoff = sc.get<int>(P.m);
+        if (!g.bits || !g.bitoff) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's bitmaps)");
     }
     CUDA_OK(row_symbolic(pool, g, prod, heavy, h, rowcnt, items, (unsigned)cap, rs, lanes));
     CUDA_OK(scan_i32_to_i64(pool, rowcnt, P.rowptrC, P.m, ctx->dflags));
@@ -1494,6 +1498,12 @@ tsg_status tsg_inject_alloc_failure(int32_t kind, int64_t countdown)
     if (kind != 0 && kind != 1) return fail(TSG_ERR_INVALID_ARG, "kind must be 0 (device pool) or 1 (pinned host)");
     if (countdown < 0) return fail(TSG_ERR_INVALID_ARG, "countdown must be >= 0");
     g_fail_alloc[kind].store(countdown, std::memory_order_relaxed);
+    return TSG_OK;
+}
+
+tsg_status tsg_inject_free_memory(int64_t bytes)
+{
+    g_free_memory.store(bytes < 0 ? -1 : bytes, std::memory_order_relaxed);
     return TSG_OK;
 }
 

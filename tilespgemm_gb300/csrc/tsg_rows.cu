@@ -171,7 +171,7 @@ k_row_products(RowArgs g, const int4 *__restrict__ ext, int *prod, int2 *rng, in
         } else {
             width = max(width, nb);
             if (p >= KEEP_BITS * (long long)nb) sb += (unsigned long long)nb;
-            si += (unsigned long long)min(p, (long long)((nb + ITEM_BLKS - 1) / ITEM_BLKS) + min(p, (long long)g.n) / ITEM_T);
+            si += (unsigned long long)item_bound(p, nb, g.n);
             if (p > LIGHT_ROW || nb > SYM_BLKS) seen |= SEEN_CUTS;
             if (p > LIGHT_MANY) seen |= SEEN_MANY;
         }

@@ -70,6 +70,18 @@ static_assert(LIGHT_BLKS * (ROW_BLK / 4) + LIGHT_ROW * 12 <= class_smem(6), "eve
 static_assert(LIGHT_ROW * 2 * 9 <= class_smem(6) && ITEM_CAP * 2 * 9 <= class_smem(6), "dense items fit");
 static_assert(ITEM_BLKS * (ROW_BLK / 4) + ITEM_CAP * 12 <= class_smem(3), "every other item fits a warp's classes");
 
+// The items of a row of p products over nb of n columns' blocks at most: its
+// entries are no more than its products or its columns.  A row that is light
+// whatever the product's size closes items at LIGHT_BLKS blocks alone.  The
+// seven lists of items are as long as these bounds' sum, 112 bytes an item.
+__host__ __device__ inline long long item_bound(long long p, int nb, int n)
+{
+    const long long span = (long long)nb * ROW_BLK, most = span < n ? span : n, z = p < most ? p : most;
+    const long long k = z <= LIGHT_MANY ? (nb + LIGHT_BLKS - 1) / LIGHT_BLKS : (nb + ITEM_BLKS - 1) / ITEM_BLKS + z / ITEM_T;
+    return p < k ? p : k;
+}
+static_assert(LIGHT_MANY <= LIGHT_ROW, "light in a large product is light in a small one");
+
 constexpr int SORT_BITS = 9, SORT_MAX = 1 << SORT_BITS;   // products of a row that is sorted at most
 constexpr int SORT_COLS = (1 << (32 - SORT_BITS)) - 1;    // C's columns up to which it is (32-bit keys)
 constexpr int SORT_NB = 80;                                // blocks of its span from which it is
