@@ -155,6 +155,11 @@ int64_t tsg_launch_count(void);
  * process instead of through the tiles: the two give the same bits, so only
  * this tells them apart (no counterpart in the reference). */
 int64_t tsg_row_path_count(void);
+
+/* Bytes of device memory the context keeps as scratch for its next tsg_spgemm
+ * or tsg_spgemm_batched: at most 4 GB, given back when any call on the device
+ * runs out of memory (no counterpart in the reference). */
+int64_t tsg_scratch_bytes(const tsg_ctx *ctx);
 void *tsg_get_stream(tsg_ctx *ctx);
 
 /* Order the context's stream after the work already queued on `stream` (a
@@ -182,7 +187,10 @@ tsg_status tsg_measure_fp64_peak(tsg_ctx *ctx, double *gflops);
  *   from a context's pool, kind 1: pinned host memory (host results and
  *   staging).  Process-wide; countdown 0 disarms it.  The call that meets the
  *   failure returns TSG_ERR_OOM, releases what it holds, and its context
- *   stays usable.  tsg_alloc_failure_pending: allocations still to go before
+ *   stays usable.  Kind 2: device memory as a full device refuses it: idle
+ *   contexts give back the scratch they keep and the allocation is tried
+ *   again; a product that still has no room is run once more without kept
+ *   scratch, through the tiles.  tsg_alloc_failure_pending: allocations still to go before
  *   the armed failure (0: none armed, or it has fired).
  * tsg_inject_check_failure: the `countdown`-th numeric step from now reports
  *   what its kernels report when an entry of C does not fit the symbolic

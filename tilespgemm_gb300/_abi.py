@@ -104,6 +104,7 @@ SIGNATURES = {
     "tsg_last_error": (C.c_char_p, []),
     "tsg_version": (C.c_char_p, []),
     "tsg_launch_count": (C.c_int64, []),
+    "tsg_scratch_bytes": (C.c_int64, [C.c_void_p]),
     "tsg_row_path_count": (C.c_int64, []),
     "tsg_pinned_cache_cap": (C.c_int64, []),
     "tsg_get_stream": (C.c_void_p, [C.c_void_p]),

@@ -99,11 +99,11 @@ void tsg::count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 // armed allocation failures per kind: the allocation that takes the count
 // from 1 to 0 fails; 0 (or below) = disarmed
-static std::atomic<long long> g_fail_alloc[2];
+static std::atomic<long long> g_fail_alloc[3];
 
 bool tsg::alloc_should_fail(int kind)
 {
-    std::atomic<long long> &c = g_fail_alloc[kind & 1];
+    std::atomic<long long> &c = g_fail_alloc[kind];
     if (c.load(std::memory_order_relaxed) <= 0) return false;
     return c.fetch_sub(1, std::memory_order_relaxed) == 1;
 }
@@ -153,6 +153,13 @@ static tsg_status fail(tsg_status st, const char *fmt, ...)
 
 // status of a failed CUDA call: out of memory is TSG_ERR_OOM, the rest TSG_ERR_CUDA
 static inline tsg_status cuda_status(cudaError_t e) { return e == cudaErrorMemoryAllocation ? TSG_ERR_OOM : TSG_ERR_CUDA; }
+
+// a CUDA call's status, for those whose failure has something to undo first
+static tsg_status cuda_result(cudaError_t e, const char *what, int line)
+{
+    return e == cudaSuccess ? TSG_OK : fail(cuda_status(e), "%s: %s (%s:%d)", what, cudaGetErrorString(e), __FILE__, line);
+}
+#define CUDA_ST(call) cuda_result((call), #call, __LINE__)
 
 #define CUDA_OK(call)                                                                                  \
     do {                                                                                               \
@@ -347,13 +354,28 @@ struct DevCSR {
     const double *val = nullptr;
 };
 
+// The process's contexts, for arenas_give_back.
+struct Contexts {
+    std::mutex mu;
+    std::vector<tsg_ctx *> all;
+};
+
+Contexts &contexts()
+{
+    static Contexts c;
+    return c;
+}
+
 // One tsg_spgemm call's use of its context's arena: empty at the start
 // (the call before is ahead of it on the context's stream), grown at the end
-// to what the call asked for.
+// to what the call asked for.  use = false, or while another thread gives the
+// arena back: everything comes from the pool.
 struct ArenaUse {
     Arena &a;
     Pool &pool;
-    ArenaUse(Arena &arena, Pool &p) : a(arena), pool(p) {
+    const bool held;
+    ArenaUse(Arena &arena, Pool &p, bool use) : a(arena), pool(p), held(use && !arena.busy.exchange(true)) {
+        if (!held) return;
         a.used = a.asked = 0;
         if (a.want > a.cap) {
             drop();
@@ -364,14 +386,21 @@ struct ArenaUse {
         }
         pool.arena = &a;
     }
+    ArenaUse(const ArenaUse &) = delete;
+    bool has() const { return held && a.cap > 0; }
     void drop() {   // back to the pool, after the work that uses it
+        if (!held) return;
         if (a.base) cudaFreeAsync(a.base, pool.stream);
+        if (a.base && pool.full) a.rest = a.last_rest = std::min(2 * a.last_rest + 1, 1023);
         a.base = nullptr;
         a.cap = a.used = 0;
     }
     ~ArenaUse() {
-        if (a.asked > a.cap && a.asked <= ARENA_MAX) a.want = a.asked;
+        if (!held) return;
+        if (a.rest > 0) --a.rest;
+        else if (a.asked > a.cap && a.asked <= ARENA_MAX) a.want = a.asked;
         pool.arena = nullptr;
+        a.busy.store(false);
     }
 };
 
@@ -1441,6 +1470,111 @@ tsg_status small_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr
 
 }  // namespace
 
+bool tsg::arenas_give_back(cudaStream_t on)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    int dev = 0;
+    if (cudaStreamIsCapturing(on, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    bool any = false;
+    Contexts &cs = contexts();
+    std::lock_guard<std::mutex> lk(cs.mu);     // none of them is destroyed meanwhile
+    for (tsg_ctx *c : cs.all) {
+        Arena &a = c->arena;
+        if (c->device != dev || a.busy.exchange(true)) continue;
+        if (a.base) {
+            // on the copy stream: the main one may be recording a graph in
+            // another thread, and no work that uses the arena is in flight
+            cudaFreeAsync(a.base, c->copy);
+            cudaStreamSynchronize(c->copy);
+            cudaMemPoolTrimTo(c->pool, 0);     // for the others' pools
+            a.base = nullptr;
+            a.cap = a.used = a.want = 0;
+            any = true;
+        }
+        a.busy.store(false);
+    }
+    cudaGetLastError();
+    return any;
+}
+
+// spgemm_call and batched_call: one attempt at the call.  kept = true: with the
+// context's arena, by rows where that pays.  A call that runs out of device
+// memory so (`spare`: there was an arena, or the row path's tables) is run once
+// more without both, with scratch that is freed as it goes: what the tiled
+// pipeline alone has room for does not fail for what speeds up others.
+namespace {
+
+tsg_status spgemm_call(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr *B, tsg_csr *C, tsg_stats *st, bool kept,
+                       bool &spare)
+{
+    Pool pool{ctx->pool, ctx->stream};
+    ArenaUse arena(ctx->arena, pool, kept);
+    PlanData P;
+    PhaseTimer tm(ctx, st && ctx->opts.phase_times);
+    int *col = nullptr;
+    double *val = nullptr;
+    EarlyOut eo;
+    tsg_status r;
+    bool emitted = false;      // col and val are C's, or freed
+    const bool by_rows = kept && !st && ctx->opts.small_path;   // rows have no statistics (of tiles and bins) to give
+    RowStart rows;
+    {
+        Scratch sc(pool);
+        r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, st != nullptr && ctx->opts.count_products, tm, true,
+                          by_rows ? &rows : nullptr);
+        if (!r && rows.take) {
+            bool taken = false;
+            r = rows_product(ctx, pool, P, rows, col, val, taken);
+            if (!r && taken) {
+                emitted = true;
+                r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st);
+            } else if (!r) {   // no room for its tables: the tiled path, from the start
+                P.release(pool);
+                P = PlanData();
+                r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, false, tm);
+            }
+        }
+        if (!emitted) {
+            if (!r && output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))   // before any work on C
+                r = fail(TSG_ERR_INT32_OVERFLOW, "C has %lld entries; int32 row pointers cannot hold them", P.nnzC);
+            if (!r) {
+                col = pool.out_n<int>(P.nnzC);
+                val = pool.out_n<double>(P.nnzC);
+                if (!col || !val) r = fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
+            }
+            if (!r && early_out_pays(P, C)) r = early_out_begin(ctx, pool, P, col, val, eo);
+            if (!r) r = plan_numeric(ctx, pool, P, P.valA, P.valB, col, val, nullptr, 0, -1, eo.on);
+            tm.mark();  // 4
+        }
+    }
+    if (!r && !emitted) {
+        fill_stats(P, st);
+        emitted = true;
+        r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st, &eo);
+    }
+    if (r) {
+        early_out_abort(ctx, pool, eo);
+        if (!emitted) { pool.free(col); pool.free(val); }
+        P.release(pool);
+        spare = pool.full && (arena.has() || by_rows);
+        if (r == TSG_ERR_OOM) arena.drop();
+        cudaStreamSynchronize(ctx->stream);
+        cudaGetLastError();
+        return r;
+    }
+    P.release(pool);
+    if (st) {
+        phase_times(ctx, st, tm);
+        st->n_syncs = P.nsync + 1;
+    }
+    return TSG_OK;
+}
+
+}  // namespace
+
 void *tsg::make_malloc_owner(void *a, void *b, void *c)
 {
     OutOwner *o = new OutOwner();
@@ -1478,6 +1612,8 @@ const char *tsg_version(void) { return "tilespgemm-gb300 0.1 (sm_103a)"; }
 
 int64_t tsg_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
+int64_t tsg_scratch_bytes(const tsg_ctx *ctx) { return ctx ? (int64_t)ctx->arena.cap : -1; }
+
 int64_t tsg_row_path_count(void) { return g_row_products.load(std::memory_order_relaxed); }
 
 int64_t tsg_pinned_cache_cap(void) { return (int64_t)pinned_cap(); }
@@ -1495,7 +1631,8 @@ tsg_status tsg_stream_wait(tsg_ctx *ctx, void *stream)
 
 tsg_status tsg_inject_alloc_failure(int32_t kind, int64_t countdown)
 {
-    if (kind != 0 && kind != 1) return fail(TSG_ERR_INVALID_ARG, "kind must be 0 (device pool) or 1 (pinned host)");
+    if (kind < 0 || kind > 2)
+        return fail(TSG_ERR_INVALID_ARG, "kind must be 0 (device pool), 1 (pinned host) or 2 (device memory full)");
     if (countdown < 0) return fail(TSG_ERR_INVALID_ARG, "countdown must be >= 0");
     g_fail_alloc[kind].store(countdown, std::memory_order_relaxed);
     return TSG_OK;
@@ -1516,7 +1653,7 @@ tsg_status tsg_inject_check_failure(int64_t countdown)
 
 int64_t tsg_alloc_failure_pending(int32_t kind)
 {
-    if (kind != 0 && kind != 1) return -1;
+    if (kind < 0 || kind > 2) return -1;
     const long long c = g_fail_alloc[kind].load(std::memory_order_relaxed);
     return c > 0 ? c : 0;
 }
@@ -1613,6 +1750,10 @@ tsg_status tsg_create(tsg_ctx **out, int device, const tsg_opts *opts)
     if (e == cudaSuccess) e = rows_init_attributes();
     if (e != cudaSuccess) return cleanup(fail(TSG_ERR_CUDA, "kernel attributes: %s", cudaGetErrorString(e)));
     noalloc_forget(device);   // tsg_tiles_to_csr_noalloc resolves its scratch address again
+    {
+        std::lock_guard<std::mutex> lk(contexts().mu);
+        contexts().all.push_back(c);
+    }
     *out = c;
     return TSG_OK;
 }
@@ -1620,6 +1761,11 @@ tsg_status tsg_create(tsg_ctx **out, int device, const tsg_opts *opts)
 tsg_status tsg_destroy(tsg_ctx *c)
 {
     if (!c) return TSG_OK;
+    {
+        std::vector<tsg_ctx *> &all = contexts().all;
+        std::lock_guard<std::mutex> lk(contexts().mu);
+        all.erase(std::remove(all.begin(), all.end(), c), all.end());
+    }
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->counted) pinned_context_leave();
@@ -1683,64 +1829,11 @@ tsg_status tsg_spgemm(tsg_ctx *ctx, tsg_op op, const tsg_csr *A, const tsg_csr *
         const tsg_status rs = small_spgemm(ctx, op, A, B, C, st, taken);
         if (taken) return rs;
     }
-    Pool pool{ctx->pool, ctx->stream};
-    ArenaUse arena(ctx->arena, pool);
-    PlanData P;
-    PhaseTimer tm(ctx, st && ctx->opts.phase_times);
-    int *col = nullptr;
-    double *val = nullptr;
-    EarlyOut eo;
-    tsg_status r;
-    {
-        Scratch sc(pool);
-        // a call without statistics (of tiles and bins) may go by rows
-        RowStart rows;
-        r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, st != nullptr && ctx->opts.count_products, tm, true,
-                          !st && ctx->opts.small_path ? &rows : nullptr);
-        if (!r && rows.take) {
-            bool taken = false;
-            r = rows_product(ctx, pool, P, rows, col, val, taken);
-            if (!r && taken) {
-                r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st);   // frees col and val on failure
-                P.release(pool);
-                return r;
-            }
-            if (!r) {   // no room for its tables: the tiled path, from the start
-                P.release(pool);
-                P = PlanData();
-                r = plan_symbolic(ctx, pool, sc, op, A, B, P, false, false, tm);
-            }
-        }
-        if (!r && output_bits(ctx, P.nnzC) == 32 && P.nnzC >= (1ll << 31))   // before any work on C
-            r = fail(TSG_ERR_INT32_OVERFLOW, "C has %lld entries; int32 row pointers cannot hold them", P.nnzC);
-        if (!r) {
-            col = pool.out_n<int>(P.nnzC);
-            val = pool.out_n<double>(P.nnzC);
-            if (!col || !val) r = fail(TSG_ERR_OOM, "device pool allocation failed for C (%lld entries)", P.nnzC);
-        }
-        if (!r && early_out_pays(P, C)) r = early_out_begin(ctx, pool, P, col, val, eo);
-        if (!r) r = plan_numeric(ctx, pool, P, P.valA, P.valB, col, val, nullptr, 0, -1, eo.on);
-        tm.mark();  // 4
-    }
-    if (r) {
-        early_out_abort(ctx, pool, eo);
-        pool.free(col); pool.free(val);
-        P.release(pool);
-        if (r == TSG_ERR_OOM) arena.drop();
-        cudaStreamSynchronize(ctx->stream);
-        cudaGetLastError();
-        return r;
-    }
-    fill_stats(P, st);
-    r = emit_output(ctx, pool, P.m, P.n, P.nnzC, P.rowptrC, col, val, C, st, &eo);
-    P.release(pool);
-    if (r) return r;
-    if (st) {
-        st->ms_total = ms_since(t0);
-        phase_times(ctx, st, tm);
-        st->n_syncs = P.nsync + 1;
-    }
-    return TSG_OK;
+    bool spare = false;
+    tsg_status r = spgemm_call(ctx, op, A, B, C, st, true, spare);
+    if (r == TSG_ERR_OOM && spare) r = spgemm_call(ctx, op, A, B, C, st, false, spare);
+    if (!r && st) st->ms_total = ms_since(t0);
+    return r;
 }
 
 // ---- plans: symbolic once, numeric many times ------------------------------
@@ -2454,28 +2547,10 @@ tsg_status pack_operands(tsg_ctx *ctx, Pool &pool, Scratch &sc, int count, const
     return TSG_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_csr *A, const tsg_csr *B,
-                              tsg_csr *C, tsg_stats *st)
+// One attempt at a batch, as spgemm_call's.
+tsg_status batched_call(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_csr *A, const tsg_csr *B, tsg_csr *C,
+                        tsg_stats *st, bool kept, bool &spare)
 {
-    if (!ctx || !C || (count > 0 && !A)) return fail(TSG_ERR_INVALID_ARG, "ctx/A/C is NULL");
-    if (count < 0) return fail(TSG_ERR_INVALID_ARG, "negative count");
-    if (op == TSG_OP_AB && count > 0 && !B) return fail(TSG_ERR_INVALID_ARG, "B is NULL for A*B");
-    if (C[0].where != TSG_MEM_HOST && C[0].where != TSG_MEM_DEVICE) return fail(TSG_ERR_INVALID_ARG, "C[0].where is not a tsg_mem");
-    if (st) memset(st, 0, sizeof(*st));
-    if (count == 0) return TSG_OK;
-    auto t0 = std::chrono::steady_clock::now();
-    CUDA_OK(cudaSetDevice(ctx->device));
-    for (int i = 0; i < count; ++i) {
-        tsg_status r = check_op(op, &A[i], op == TSG_OP_AB ? &B[i] : nullptr);
-        if (r) return r;
-        if (A[i].where != A[0].where || (op == TSG_OP_AB && B[i].where != A[0].where))
-            return fail(TSG_ERR_INVALID_ARG, "all batch operands must be host, or all device");
-        if (A[i].nnz > 0 && !A[i].val) return fail(TSG_ERR_INVALID_ARG, "instance %d has no values", i);
-    }
     // layout: rows of A (and C), columns of A (= rows of B), columns of B (and C)
     std::vector<long long> roff(count), koff(count), noff(count);
     long long M = 0, K = 0, N = 0;
@@ -2486,12 +2561,14 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         noff[i] = N; N += round16(ni);
     }
     Pool pool{ctx->pool, ctx->stream};
-    ArenaUse arena(ctx->arena, pool);
+    ArenaUse arena(ctx->arena, pool, kept);
     PlanData P;
     PhaseTimer tm(ctx, st && ctx->opts.phase_times);
     int *col = nullptr;
     double *val = nullptr;
     tsg_status r;
+    RowStart rows;
+    const bool by_rows = kept && !st && ctx->opts.small_path;
     {
         Scratch sc(pool);
         CUDA_OK(cudaMemsetAsync(ctx->dflags, 0, sizeof(int) * FLAG_COUNT, ctx->stream));
@@ -2499,9 +2576,8 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
         r = pack_operands(ctx, pool, sc, count, A, roff, op == TSG_OP_AAT ? koff : (op == TSG_OP_AA ? roff : koff),
                           M, op == TSG_OP_AA ? M : K, pA);
         if (!r && op == TSG_OP_AB) r = pack_operands(ctx, pool, sc, count, B, koff, noff, K, N, pB);
-        RowStart rows;
         if (!r) r = plan_symbolic(ctx, pool, sc, op, &pA, op == TSG_OP_AB ? &pB : nullptr, P, false, st != nullptr && ctx->opts.count_products, tm,
-                                  false, !st && ctx->opts.small_path ? &rows : nullptr);
+                                  false, by_rows ? &rows : nullptr);
         // C's column offset of each packed tile-row's instance: the numeric
         // step writes C_i's columns already rebased
         long long rpn = 0;
@@ -2518,7 +2594,7 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
             d_trc = sc.get<int>((long long)trc.size());
             if (!d_trc) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch layout)");
         }
-        if (!r) CUDA_OK(cudaMemcpyAsync(d_trc, trc.data(), sizeof(int) * trc.size(), cudaMemcpyHostToDevice, ctx->stream));
+        if (!r) r = CUDA_ST(cudaMemcpyAsync(d_trc, trc.data(), sizeof(int) * trc.size(), cudaMemcpyHostToDevice, ctx->stream));
         bool taken = false;
         std::vector<int> base;
         if (!r && rows.take) {
@@ -2533,7 +2609,7 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
             }
             int *d_base = sc.get<int>((long long)base.size());
             if (!d_base) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch layout)");
-            if (!r) CUDA_OK(cudaMemcpyAsync(d_base, base.data(), sizeof(int) * base.size(), cudaMemcpyHostToDevice, ctx->stream));
+            if (!r) r = CUDA_ST(cudaMemcpyAsync(d_base, base.data(), sizeof(int) * base.size(), cudaMemcpyHostToDevice, ctx->stream));
             rb.base = d_base; rb.coloff = d_trc;
             if (!r) r = rows_product(ctx, pool, P, rows, col, val, taken, &rb);
             if (!r && !taken) {
@@ -2560,17 +2636,15 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
             ebase = sc.get<long long>(count);
             UnpackDesc *dud = sc.get<UnpackDesc>(count);
             if (!rp_out || !ebase || !dud) r = fail(TSG_ERR_OOM, "device pool allocation failed (batch outputs)");
-            if (!r) {
-                CUDA_OK(cudaMemcpyAsync(dud, ud.data(), sizeof(UnpackDesc) * (size_t)count, cudaMemcpyHostToDevice, ctx->stream));
-                CUDA_OK(batch_unpack(pool, dud, count, P.rowptrC, rp_out, bits, ebase));
-            }
+            if (!r) r = CUDA_ST(cudaMemcpyAsync(dud, ud.data(), sizeof(UnpackDesc) * (size_t)count, cudaMemcpyHostToDevice, ctx->stream));
+            if (!r) r = CUDA_ST(batch_unpack(pool, dud, count, P.rowptrC, rp_out, bits, ebase));
         }
         std::vector<long long> eb(count);
+        if (!r) r = CUDA_ST(cudaMemcpyAsync(eb.data(), ebase, sizeof(long long) * (size_t)count, cudaMemcpyDeviceToHost, ctx->stream));
+        if (!r) r = CUDA_ST(cudaStreamSynchronize(ctx->stream));
+        int hflags[FLAG_COUNT] = {};
+        if (!r) r = CUDA_ST(cudaMemcpy(hflags, ctx->dflags, sizeof(hflags), cudaMemcpyDeviceToHost));
         if (!r) {
-            CUDA_OK(cudaMemcpyAsync(eb.data(), ebase, sizeof(long long) * (size_t)count, cudaMemcpyDeviceToHost, ctx->stream));
-            CUDA_OK(cudaStreamSynchronize(ctx->stream));
-            int hflags[FLAG_COUNT];
-            CUDA_OK(cudaMemcpy(hflags, ctx->dflags, sizeof(hflags), cudaMemcpyDeviceToHost));
             if (hflags[FLAG_BAD_INPUT]) r = fail(TSG_ERR_BAD_INPUT, "an instance's row pointer or column index is out of range");
             else if (hflags[FLAG_INTERNAL]) r = fail(TSG_ERR_CUDA, "internal bound check failed on the device");
         }
@@ -2630,6 +2704,8 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
     if (r) {
         pool.free(col); pool.free(val);
         P.release(pool);
+        spare = pool.full && (arena.has() || by_rows);
+        if (r == TSG_ERR_OOM) arena.drop();
         cudaStreamSynchronize(ctx->stream);
         cudaGetLastError();
         return r;
@@ -2637,11 +2713,37 @@ tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_
     fill_stats(P, st);
     P.release(pool);
     cudaStreamSynchronize(ctx->stream);
-    if (st) {
-        st->ms_total = ms_since(t0);
-        phase_times(ctx, st, tm);
-    }
+    if (st) phase_times(ctx, st, tm);
     return TSG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+tsg_status tsg_spgemm_batched(tsg_ctx *ctx, tsg_op op, int32_t count, const tsg_csr *A, const tsg_csr *B,
+                              tsg_csr *C, tsg_stats *st)
+{
+    if (!ctx || !C || (count > 0 && !A)) return fail(TSG_ERR_INVALID_ARG, "ctx/A/C is NULL");
+    if (count < 0) return fail(TSG_ERR_INVALID_ARG, "negative count");
+    if (op == TSG_OP_AB && count > 0 && !B) return fail(TSG_ERR_INVALID_ARG, "B is NULL for A*B");
+    if (C[0].where != TSG_MEM_HOST && C[0].where != TSG_MEM_DEVICE) return fail(TSG_ERR_INVALID_ARG, "C[0].where is not a tsg_mem");
+    if (st) memset(st, 0, sizeof(*st));
+    if (count == 0) return TSG_OK;
+    auto t0 = std::chrono::steady_clock::now();
+    CUDA_OK(cudaSetDevice(ctx->device));
+    for (int i = 0; i < count; ++i) {
+        tsg_status r = check_op(op, &A[i], op == TSG_OP_AB ? &B[i] : nullptr);
+        if (r) return r;
+        if (A[i].where != A[0].where || (op == TSG_OP_AB && B[i].where != A[0].where))
+            return fail(TSG_ERR_INVALID_ARG, "all batch operands must be host, or all device");
+        if (A[i].nnz > 0 && !A[i].val) return fail(TSG_ERR_INVALID_ARG, "instance %d has no values", i);
+    }
+    bool spare = false;
+    tsg_status r = batched_call(ctx, op, count, A, B, C, st, true, spare);
+    if (r == TSG_ERR_OOM && spare) r = batched_call(ctx, op, count, A, B, C, st, false, spare);
+    if (!r && st) st->ms_total = ms_since(t0);
+    return r;
 }
 
 }  // extern "C"

@@ -9,6 +9,7 @@
 //   C tiles       crp (int64, blkm+1), ccol (int32), cmask (uint16, 16 per tile)
 //   C CSR         rowptr (int64, m+1), col (int32), val (f64)
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -128,7 +129,8 @@ namespace tsg {
 void count_launch();
 
 // Fault injection (tsg_inject_alloc_failure): true when this allocation of
-// `kind` (0: device pool, 1: pinned host) is the one armed to fail.
+// `kind` (0: device pool, 1: pinned host, 2: device memory that is full) is
+// the one armed to fail.
 bool alloc_should_fail(int kind);
 
 // Scratch of a context's calls, kept between them: one block, handed out from
@@ -137,14 +139,26 @@ bool alloc_should_fail(int kind);
 // time nor the pool's searches among C's long-lived blocks, whose gaps had
 // made it remap memory within a call (96^3 27-point stencil: 3.75 or 4.65 ms
 // a call, by the order in which the caller freed earlier results).  At most
-// ARENA_MAX; what does not fit comes from the pool.
+// ARENA_MAX; what does not fit comes from the pool.  No work that uses it is
+// in flight outside of a call, so whoever runs out of device memory may give
+// it back in between (arenas_give_back).
 constexpr size_t ARENA_MAX = (size_t)4 << 30;
 struct Arena {
     char *base = nullptr;
     size_t cap = 0, used = 0;
-    size_t asked = 0;    // bytes this call asked for
-    size_t want = 0;     // the block the next call starts with, if larger
+    size_t asked = 0;            // bytes this call asked for
+    size_t want = 0;             // the block the next call starts with, if larger
+    // calls to go without growing, after a call that ran out of memory with it
+    // had to be run again: twice as many each time, so that calls on a device
+    // that stays full do not run twice over and over
+    int rest = 0, last_rest = 0;
+    std::atomic<bool> busy{false};   // a call uses it, or it is being given back
 };
+
+// Gives every context's idle arena on the current device back to the driver;
+// true if there was one.  `on`: the stream the caller allocates on (nothing is
+// done while it records a graph).
+bool arenas_give_back(cudaStream_t on);
 
 // Stream-ordered allocations from the context's memory pool.  The pool keeps
 // freed memory cached (release threshold = max), so steady-state calls do no
@@ -156,6 +170,7 @@ struct Pool {
     cudaStream_t stream = nullptr;
     cudaError_t err = cudaSuccess;
     Arena *arena = nullptr;
+    bool full = false;           // an allocation failed because the device's memory was full
     void *alloc(size_t bytes) {
         if (!arena) return out(bytes);
         const size_t need = (bytes + 255) & ~(size_t)255;
@@ -170,9 +185,17 @@ struct Pool {
         if (bytes == 0) bytes = 16;
         if (alloc_should_fail(0)) { err = cudaErrorMemoryAllocation; return nullptr; }
         void *p = nullptr;
-        cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+        cudaError_t e = take(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {    // what idle arenas hold is the callers', too
+            cudaGetLastError();
+            if (arenas_give_back(stream)) e = take(p, bytes);
+            full |= e == cudaErrorMemoryAllocation;
+        }
         if (e != cudaSuccess) { err = e; cudaGetLastError(); return nullptr; }
         return p;
+    }
+    cudaError_t take(void *&p, size_t bytes) {
+        return alloc_should_fail(2) ? cudaErrorMemoryAllocation : cudaMallocFromPoolAsync(&p, bytes, pool, stream);
     }
     template <class T> T *alloc_n(long long n) { return static_cast<T *>(alloc(sizeof(T) * (size_t)(n > 0 ? n : 1))); }
     template <class T> T *out_n(long long n) { return static_cast<T *>(out(sizeof(T) * (size_t)(n > 0 ? n : 1))); }
