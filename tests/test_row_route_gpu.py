@@ -137,3 +137,40 @@ def test_items_of_light_rows_fit_their_bound(rctx):  # noqa: F811
         C, went = _went(lambda: rctx.spgemm(A, B, op="AB"))
         assert went == 1
         _check(C, O.spgemm(A, B))
+
+
+def _spaced(m, n, lens, seed):
+    """m rows of the given lengths over n columns: one random column of each of
+    so many equal parts of them, so that hardly two share a tile."""
+    from tilespgemm_gb300.api import CSR
+    rng = np.random.default_rng(seed)
+    lens = np.resize(np.asarray(lens, np.int64), m)
+    rp = np.zeros(m + 1, np.int64)
+    np.cumsum(lens, out=rp[1:])
+    part = n // np.maximum(lens, 1)
+    at = np.arange(rp[-1]) - np.repeat(rp[:-1], lens)
+    wide = np.repeat(part, lens)
+    col = at * wide + (rng.random(at.size) * wide).astype(np.int64)
+    return CSR(m, n, rp, col.astype(np.int32), rng.uniform(-1.0, 1.0, int(rp[-1])))
+
+
+def _band(n, h, seed):
+    from tilespgemm_gb300.api import CSR
+    c = np.arange(n)[:, None] + np.arange(-h, h + 1)[None, :]
+    ok = (c >= 0) & (c < n)
+    rp = np.zeros(n + 1, np.int64)
+    np.cumsum(ok.sum(1), out=rp[1:])
+    return CSR(n, n, rp, c[ok].astype(np.int32), np.random.default_rng(seed).uniform(-1.0, 1.0, int(rp[-1])))
+
+
+@pytest.mark.parametrize("m,clustered,rows", [(65536, True, 1), (65537, True, 0), (65537, False, 1)])
+def test_many_clustered_rows_go_by_tiles(rctx, ctx, m, clustered, rows):  # noqa: F811
+    """Under 24 M products, on both sides of 65,536 rows: there the rows' fixed
+    cost counts, and tiles that hold several entries a row are cheaper."""
+    A = _band(m, 6, 95) if clustered else _spaced(m, m, [13], 96)
+    op = "AA"
+    C, went = _went(lambda: rctx.spgemm(A, op=op))
+    assert went == rows
+    D, none = _went(lambda: ctx.spgemm(A, op=op))
+    assert none == 0
+    _check(C, (np.asarray(D.rowptr, np.int64), D.col, D.val))

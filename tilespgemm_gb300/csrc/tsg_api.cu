@@ -636,11 +636,16 @@ tsg_status stage_into_plan(tsg_ctx *ctx, Pool &pool, PlanData &P, const tsg_csr 
 
 // Whether the row path (tsg_rows.cu) takes a product: `products` is the
 // sampled estimate, runs the operands' tile runs.
-// - Under 24 M products the tiled path's 25 launches and half-empty kernels
-//   cost more than its tiles save (31^3 27-point stencil, 19 M: 455 us tiled,
-//   383 by rows; R-MAT 2^12: 1,180 and 440); large ones only with fewer than
-//   1.5 entries a tile run (200,000 rows of 20 in a band of +-300, 1.25 a run:
-//   1,447 us tiled, 1,295 by rows; +-100, 1.84: 1,066 and 1,279).
+// - Under 24 M products and 65,536 rows the tiled path's 25 launches and
+//   half-empty kernels cost more than its tiles save (31^3 27-point stencil,
+//   19 M: 455 us tiled, 383 by rows; R-MAT 2^12: 1,180 and 440; the line is
+//   where bands cross: A*A of 50,000 rows +-6 330 and 329, 65,000 354 and 386,
+//   but A*A^T, with another conversion, 517 and 491).
+// - Larger ones only with fewer than 1.5 entries a tile run (200,000 rows of 20
+//   in a band of +-300, 1.25 a run: 1,447 us tiled, 1,295 by rows; +-100, 1.84:
+//   1,066 and 1,279; 100,000 rows of 15 in a band of +-7, 8.9 a run: 465 and
+//   558, +-80, 1.72: 558 and 607, +-160, 1.31: 620 and 611, +-20,000: 4,614
+//   and 1,173).
 // - A row costs the row path a few microseconds of a CTA whatever it holds:
 //   rows of under 128 products go by tiles when there are many (96^3 7-point
 //   stencil, 48 a row: 2.0 ms tiled, 5.2 by rows).
@@ -648,9 +653,8 @@ constexpr long long ROW_PRODUCTS = 24000000;
 constexpr int ROW_FEW = 65536;
 bool rows_pay(const PlanData &P, long long products, long long runsA, long long runsB)
 {
-    const bool full = products >= 128ll * P.m;
-    if (products <= ROW_PRODUCTS) return full || P.m <= ROW_FEW;
-    return full && 2 * P.nnzA < 3 * runsA && 2 * P.nnzB < 3 * runsB;
+    if (products <= ROW_PRODUCTS && P.m <= ROW_FEW) return true;
+    return products >= 128ll * P.m && 2 * P.nnzA < 3 * runsA && 2 * P.nnzB < 3 * runsB;
 }
 
 // Symbolic phase: staging, A^T for A*A^T, tiles, step 1, step 2 (two host waits).
