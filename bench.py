@@ -515,23 +515,23 @@ def run_batched(args) -> None:
 
 
 def link_gbs() -> dict:
-    """Host-link bandwidth of this machine: one 2 GiB pinned copy each way, three
-    times, CUDA events (the link bounds every host-memory result)."""
+    """Host-link bandwidth of this machine: the best of eight 2 GiB pinned copies
+    each way, timed one by one with CUDA events (the link bounds every
+    host-memory result; a mean would carry whatever else the host did)."""
     import torch
     n = 1 << 31
     h = torch.empty(n, dtype=torch.uint8).pin_memory()
     d = torch.empty(n, dtype=torch.uint8, device="cuda")
     out = {}
     for name, dst, src in (("h2d", d, h), ("d2h", h, d)):
-        dst.copy_(src, non_blocking=True)
-        torch.cuda.synchronize()
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        for _ in range(3):
+        out[name] = 0.0
+        for _ in range(9):                      # the first warms up
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
             dst.copy_(src, non_blocking=True)
-        e1.record()
-        e1.synchronize()
-        out[name] = 3 * n / (e0.elapsed_time(e1) * 1e6)
+            e1.record()
+            e1.synchronize()
+            out[name] = max(out[name], n / (e0.elapsed_time(e1) * 1e6))
     del h, d
     return out
 
