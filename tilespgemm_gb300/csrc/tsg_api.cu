@@ -657,8 +657,6 @@ bool rows_pay(const PlanData &P, long long products, long long runsA, long long 
     return products >= 128ll * P.m && 2 * P.nnzA < 3 * runsA && 2 * P.nnzB < 3 * runsB;
 }
 
-// Symbolic phase: staging, A^T for A*A^T, tiles, step 1, step 2 (two host waits).
-// `keep` = the plan outlives the call (device operands are copied).
 // The row path's start: its per-row arrays and what row_products found.
 struct RowStart {
     bool take = false;       // the staged operands qualify for the row path
@@ -671,9 +669,9 @@ struct RowStart {
 RowArgs row_args(const PlanData &P)
 {
     RowArgs g;
-    g.m = P.m; g.k = P.k; g.n = P.n; g.nblk = ceil_div_i(P.n, ROW_BLK);
+    g.m = P.m; g.k = P.k; g.n = P.n;
     g.rpA = P.rpA; g.rpB = P.rpB; g.colA = P.colA; g.colB = P.colB; g.valA = P.valA; g.valB = P.valB;
-    g.width = g.nblk;
+    g.width = ceil_div_i(P.n, ROW_BLK);
     g.sort_max = P.n <= SORT_COLS ? SORT_MAX : 0;
     return g;
 }
@@ -691,6 +689,8 @@ tsg_status row_count(tsg_ctx *ctx, Pool &pool, Scratch &sc, const PlanData &P, R
     return TSG_OK;
 }
 
+// Symbolic phase: staging, A^T for A*A^T, tiles, step 1, step 2 (two host waits).
+// `keep` = the plan outlives the call (device operands are copied).
 // rows (optional): the caller can take the row path; rows->take is set when the
 // staged operands qualify for it, and then nothing but the staging is done.
 tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const tsg_csr *A, const tsg_csr *B,
@@ -748,9 +748,15 @@ tsg_status plan_symbolic(tsg_ctx *ctx, Pool &pool, Scratch &sc, tsg_op op, const
             CUDA_OK(aux_rows_increasing(pool, P.rpB, P.colB, P.k, P.n, P.nnzB, rs + ST_BUNSORTED, rs + ST_TILESB));
             // where the row path is likely its products are counted at once,
             // which saves the sample and a wait (31^3 27-point stencil 362 -> 348 us,
-            // R-MAT 2^12 x 8 A*A^T 395 -> 371); elsewhere the sample is cheaper,
-            // and needless where the averages, which skew only adds to, put the
-            // products past both lines (96^3 27-point stencil 3,830 -> 3,774 us)
+            // R-MAT 2^12 x 8 A*A^T 395 -> 371); elsewhere the sample is cheaper.
+            // It is left out where the mean row lengths put the products past
+            // both lines, and the tile runs alone decide.  The mean is a lower
+            // bound for A*A^T only: elsewhere A may meet B's short rows.  Rows
+            // are still the better way then where entries lie alone (rows of 0
+            // to 3 met among rows of 400, uniform: 0.3 to 0.6 ms by rows, 2.5 to
+            // 31 by tiles) and near even at 1.4 entries a run (7-point rows met
+            // among rows of 57, 48 products a row: 96^3 5.8 ms by rows, 4.8 by
+            // tiles, 48^3 0.66 and 0.79)
             const double mean = (double)P.nnzA * (double)P.nnzB / (double)P.k;
             const bool ahead = P.m <= ROW_FEW && mean <= (double)ROW_PRODUCTS;
             const bool plain = mean > (double)ROW_PRODUCTS && mean >= 128.0 * P.m;
@@ -1162,7 +1168,7 @@ tsg_status rows_product(tsg_ctx *ctx, Pool &pool, PlanData &P, RowStart &start, 
     // a small product decide (R-MAT 2^12 A*A^T: 430 us, 509 with 64; 31^3
     // stencil, 27 each: 383 us by warps, 711 by CTAs), from 64 on where the
     // SMs are full (512 mixed products: 30.7 ms with 64, 36.6 with 32, 39.1 with 200)
-    g.each = h.products > 24000000 ? 64.0f : 32.0f;
+    g.each = (long long)h.products > ROW_PRODUCTS ? 64.0f : 32.0f;
     if (!items) return fail(TSG_ERR_OOM, "device pool allocation failed (row path's items)");
     if (h.blocks < (1ull << 31) && table_fits(128ll * (long long)h.blocks)) {   // the rows' bitmaps, kept for the numeric pass
         g.bits = sc.get<unsigned>(32ll * (long long)h.blocks);

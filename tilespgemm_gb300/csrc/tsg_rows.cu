@@ -65,10 +65,13 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 // Rows sorted in place of a bitmap: the bitmap costs by the row's blocks, the
-// sort by its products.  The line lies between spans that were measured, call
-// with bitmaps / sorted: 64 blocks (R-MAT 2^16 x 12 A*A) 3,008 / 3,155 us, 32
-// (R-MAT 2^15 x 16 A*A^T) 2,229 / 2,311, 98 (uniform, 192 products a row)
-// 2,083 / 727, 256 (R-MAT 2^18 x 16) 35,674 / 35,066.
+// sort by its products, but the line looks at the blocks alone, where R-MAT
+// graphs' rows turn.  Call with bitmaps / sorted: 32 blocks (R-MAT 2^15 x 16
+// A*A^T) 2,229 / 2,311 us, 64 (2^16 x 12 A*A) 3,008 / 3,155, 256 (2^18 x 16)
+// 35,674 / 35,066.  Uniform rows would gain by the sort from further down:
+// 120,000 of 192 products over 20 blocks 832 / 519 us, 59 1,290 / 520, 79 1,834 /
+// 517, 98 1,986 / 513; of 484 products 1,132 / 1,274, 2,101 / 1,293, 2,238 / 1,297
+// and 2,401 / 1,297.
 __device__ __forceinline__ bool sorted_row(const RowArgs &g, long long p, int nb)
 {
     return p > 0 && p <= g.sort_max && nb >= SORT_NB;

@@ -87,7 +87,7 @@ constexpr int SORT_COLS = (1 << (32 - SORT_BITS)) - 1;    // C's columns up to w
 constexpr int SORT_NB = 80;                                // blocks of its span from which it is
 
 struct RowArgs {
-    int m = 0, k = 0, n = 0, nblk = 0;
+    int m = 0, k = 0, n = 0;
     const long long *rpA = nullptr, *rpB = nullptr;
     const int *colA = nullptr, *colB = nullptr;
     const double *valA = nullptr, *valB = nullptr;
