@@ -363,7 +363,7 @@ def run_ours(args) -> None:
     fp64 = ctypes.c_double(0.0)
     _abi.check(lib.tsg_measure_fp64_peak(ctx.handle, ctypes.byref(fp64)))
     # the small-product path has no phase events: its dominant kernel
-    # (k_small_fill) is taken with the call's time and the call's bytes
+    # (k_small_fill_one) is taken with the call's time and the call's bytes
     small = bool(phases[-1].get("small_path", 0))
     ab = algorithmic_bytes(A, B, nnz_c)
     ms_num = ms if small else statistics.mean(p["ms_step3"] for p in phases)
@@ -371,7 +371,7 @@ def run_ours(args) -> None:
     achieved = kbytes / (ms_num * 1e6)
     traffic = None if small else load_traffic(args.workload)
     roofline = {
-        "kernel": ("k_small_fill (small-product path, the whole call: count pass skipped on a repeated shape)"
+        "kernel": ("k_small_fill_one (small-product path, the whole call: count pass skipped on a repeated shape)"
                    if small else "k_numeric_smem (step 3: FP64 accumulation + CSR write)"),
         "bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
         "frac": (achieved / hbm_peak) if hbm_peak else None,
