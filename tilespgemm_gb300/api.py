@@ -65,12 +65,12 @@ class CSR:
         return CSR(self.m, self.n, torch.as_tensor(np.asarray(self.rowptr)).to(dev),
                    torch.as_tensor(np.asarray(self.col)).to(dev), torch.as_tensor(np.asarray(self.val)).to(dev))
 
-    def _tsg(self, ctx_handle=None, wait: bool = True) -> tuple[_abi.tsg_csr, list]:
+    def _tsg(self, ctx_handle=None, unwaited: set | None = None) -> tuple[_abi.tsg_csr, list]:
         """tsg_csr view of this matrix plus the objects that must stay alive.
         Device tensors: the context's stream (ctx_handle) is ordered after
         torch's current stream without blocking; without a context the host
-        waits for torch's stream, which copies strided tensors here (wait
-        False: the caller does, behind the last of its views)."""
+        waits for torch's stream, which copies strided tensors here (unwaited:
+        the device goes there, and the caller waits behind its last view)."""
         s = _abi.tsg_csr()
         s.m, s.n = int(self.m), int(self.n)
         keep: list = []
@@ -88,7 +88,9 @@ class CSR:
             s.nnz = col.numel()
             if ctx_handle:
                 check(lib().tsg_stream_wait(ctx_handle, torch.cuda.current_stream(rp.device).cuda_stream))
-            elif wait:
+            elif unwaited is not None:
+                unwaited.add(rp.device)
+            else:
                 torch.cuda.current_stream(rp.device).synchronize()
         else:
             rp = np.asarray(self.rowptr)
@@ -108,18 +110,16 @@ class CSR:
         return s, keep
 
 
-def _tsg_list(Xs: list, n: int) -> tuple[Any, list, set]:
-    """tsg_csr views of Xs in one array of n, the objects that must stay
-    alive, and the devices whose torch streams the caller has to wait for."""
+def _tsg_list(Xs: list, n: int, unwaited: set) -> tuple[Any, list]:
+    """tsg_csr views of Xs in one array of n and the objects that must stay
+    alive; the devices whose torch streams the caller has to wait for go to
+    unwaited."""
     arr = (_abi.tsg_csr * max(n, 1))()
     keep: list = []
-    devices = set()
     for i, X in enumerate(Xs):
-        arr[i], k = X._tsg(wait=False)
+        arr[i], k = X._tsg(unwaited=unwaited)
         keep.append(k)
-        if X.on_device:
-            devices.add(k[0].device)
-    return arr, keep, devices
+    return arr, keep
 
 
 def _wait_torch(devices: set) -> None:
@@ -432,11 +432,11 @@ class Context:
         """C_i = op(A_i, B_i) for all instances in one pipeline pass (tsg_spgemm_batched);
         returns OwnedCSR views that share one allocation."""
         n = len(As)
-        a, keep_a, devices = _tsg_list(As, n)
+        devices: set = set()
+        a, keep_a = _tsg_list(As, n, devices)
         b_ptr, keep_b = None, None
         if Bs is not None:
-            b_ptr, keep_b, more = _tsg_list(Bs, n)
-            devices |= more
+            b_ptr, keep_b = _tsg_list(Bs, n, devices)
         _wait_torch(devices)      # once, behind the copies of every strided tensor
         c = (_abi.tsg_csr * max(n, 1))()
         c[0].where = _abi.MEM_DEVICE if out == "device" else _abi.MEM_HOST

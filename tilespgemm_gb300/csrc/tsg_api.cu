@@ -49,7 +49,8 @@ cudaError_t aux_rows_increasing(Pool &pool, const long long *rp, const int *col,
 cudaError_t aux_run_sample(Pool &pool, const int *col, long long nnz, unsigned long long *runs);
 cudaError_t aux_copy_scalars(Pool &pool, const long long *a, long long *da, const int *b, long long *db,
                              const int *c, long long *dc);
-cudaError_t aux_rowptr_narrow(Pool &pool, const long long *in, int *out, long long n);
+cudaError_t aux_rowptr_narrow(Pool &pool, const long long *in, int *out, long long n, const int *flags = nullptr,
+                              int *host_flags = nullptr);
 // the device Matrix Market reader (tsg_mtx_dev.cu)
 cudaError_t mtx_lines(Pool &pool, const char *text, long long n, long long *&ends, long long &lines, int *flags);
 cudaError_t mtx_parse(Pool &pool, const char *text, const long long *ends, long long lines, int kind, long long M,
@@ -934,18 +935,23 @@ void fill_stats(const PlanData &P, tsg_stats *st)
 }
 
 // C's row pointers for the caller (int64 copied, or narrowed to int32), on
-// the main stream
-cudaError_t output_rowptr(tsg_ctx *ctx, Pool &pool, int m, int bits, const long long *rowptr, void *&rp_dev)
+// the main stream; check: the flags go to their mirror too (flags_arrived),
+// with the narrowing kernel where there is one
+cudaError_t output_rowptr(tsg_ctx *ctx, Pool &pool, int m, int bits, const long long *rowptr, void *&rp_dev, bool check)
 {
     if (bits == 32) {
         int *rp32 = pool.out_n<int>(m + 1);
         rp_dev = rp32;
-        return rp32 ? aux_rowptr_narrow(pool, rowptr, rp32, m + 1) : cudaErrorMemoryAllocation;
+        if (!rp32) return cudaErrorMemoryAllocation;
+        return aux_rowptr_narrow(pool, rowptr, rp32, m + 1, check ? ctx->dflags : nullptr,
+                                 reinterpret_cast<int *>(ctx->hstat + ST_HFLAGS));
     }
     long long *rp64 = pool.out_n<long long>(m + 1);
     rp_dev = rp64;
-    return rp64 ? cudaMemcpyAsync(rp64, rowptr, sizeof(long long) * (size_t)(m + 1), cudaMemcpyDeviceToDevice, ctx->stream)
-                : cudaErrorMemoryAllocation;
+    if (!rp64) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMemcpyAsync(rp64, rowptr, sizeof(long long) * (size_t)(m + 1), cudaMemcpyDeviceToDevice,
+                                          ctx->stream);
+    return e == cudaSuccess && check ? flags_down(ctx) : e;
 }
 
 int output_bits(const tsg_ctx *ctx, long long nnzC)
@@ -988,7 +994,7 @@ tsg_status early_out_begin(tsg_ctx *ctx, Pool &pool, PlanData &P, int *col, doub
     eo.hval = pinned_get(ctx, eo.vb);
     if (!eo.hrp || !eo.hcol || !eo.hval) return fail(TSG_ERR_OOM, "pinned host memory for C");
     eo.on = true;
-    CUDA_OK(output_rowptr(ctx, pool, P.m, eo.bits, P.rowptrC, eo.rp_dev));
+    CUDA_OK(output_rowptr(ctx, pool, P.m, eo.bits, P.rowptrC, eo.rp_dev, false));   // the numeric step is still to come
     NumericArgs na = numeric_args(ctx, P, P.valA, P.valB, col, val, nullptr);
     CUDA_OK(numeric_cols(pool, na));
     CUDA_OK(cudaEventRecord(ctx->cols_ev, ctx->stream));
@@ -1061,13 +1067,12 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
     o->where = C->where;
     C->m = m; C->n = n; C->nnz = nnzC; C->rowptr_bits = bits;
     void *rp_dev = nullptr;
-    cudaError_t e = output_rowptr(ctx, pool, m, bits, rowptr, rp_dev);
+    cudaError_t e = output_rowptr(ctx, pool, m, bits, rowptr, rp_dev, !checked);
     if (C->where == TSG_MEM_DEVICE) {
         o->blocks.push_back({rp_dev, 0});
         o->blocks.push_back({col, 0});
         o->blocks.push_back({val, 0});
         C->row_ptr = rp_dev; C->col = col; C->val = val;
-        if (e == cudaSuccess && !checked) e = flags_down(ctx);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     } else {
         auto t_d2h = std::chrono::steady_clock::now();
@@ -1079,7 +1084,6 @@ tsg_status emit_output(tsg_ctx *ctx, Pool &pool, int m, int n, long long nnzC, c
         if (e == cudaSuccess && nnzC > 0) e = cudaMemcpyAsync(hcol, col, cb, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess && nnzC > 0) e = cudaMemcpyAsync(hval, val, vb, cudaMemcpyDeviceToHost, ctx->stream);
         pool.free(rp_dev); pool.free(col); pool.free(val);
-        if (e == cudaSuccess && !checked) e = flags_down(ctx);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (hrp) o->blocks.push_back({hrp, rpb});
         if (hcol) o->blocks.push_back({hcol, cb});

@@ -120,10 +120,13 @@ __global__ void k_copy_scalars(const long long *a, long long *da, const int *b, 
     if (threadIdx.x == 0) { *da = *a; *db = *b; *dc = *c; }
 }
 
-__global__ void k_rowptr_narrow(const long long *in, int *out, long long n)
+// flags (optional): the device's flags go to host_flags (pinned), which the
+// call's last wait then covers; a copy of their own cost 5 us of a call
+__global__ void k_rowptr_narrow(const long long *in, int *out, long long n, const int *flags, int *host_flags)
 {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i < n) out[i] = (int)in[i];
+    if (flags && i < FLAG_COUNT) host_flags[i] = flags[i];
 }
 
 // ---- C tiles from C's CSR ------------------------------------------------
@@ -500,10 +503,10 @@ cudaError_t batch_unpack(Pool &pool, const UnpackDesc *d_desc, int count, const 
     return cudaGetLastError();
 }
 
-cudaError_t aux_rowptr_narrow(Pool &pool, const long long *in, int *out, long long n)
+cudaError_t aux_rowptr_narrow(Pool &pool, const long long *in, int *out, long long n, const int *flags, int *host_flags)
 {
     if (n <= 0) return cudaSuccess;
-    { k_rowptr_narrow<<<(unsigned)((n + 255) / 256), 256, 0, pool.stream>>>(in, out, n); ::tsg::count_launch(); }
+    { k_rowptr_narrow<<<(unsigned)((n + 255) / 256), 256, 0, pool.stream>>>(in, out, n, flags, host_flags); ::tsg::count_launch(); }
     return cudaGetLastError();
 }
 
